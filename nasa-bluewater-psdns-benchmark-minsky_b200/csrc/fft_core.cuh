@@ -8,14 +8,27 @@
 // Algorithm: Stockham auto-sort with mixed register radices.  A line of N
 // points is split into passes of radix R_p (product = N).  In every pass each
 // thread owns E/R_p butterflies of radix R_p whose operands it holds in
-// registers; the radix-R kernels are unrolled at compile time with constant
-// twiddles.  Between passes data goes through shared memory in place: all
-// operands are read, the block synchronises, then all results are written.
-// Shared-memory element i of a line lives at pad(i) = i + i/32, which keeps
-// the strided writes of the first pass from serialising on one bank.  The
-// inter-pass twiddles of pass p are stored as a table [r][k] (k = j mod Ns)
-// so that consecutive threads read consecutive words.
+// registers; the radix-R kernels are unrolled at compile time.  Between passes
+// data goes through shared memory in place: all operands are read, the block
+// synchronises, then all results are written.  Shared-memory element i of a
+// line lives at pad(i) = i + i/32, which keeps the strided writes of the first
+// pass from serialising on one bank.
+//
+// What bounds the transforms inside the kernels is the number of instructions
+// issued, not the FMA pipe (the x chain issued 0.59 per cycle and scheduler at
+// 40% of that pipe), so the arithmetic is arranged for few instructions:
+//  * Complex sums, and the sums of a twiddled butterfly, are packed FP32 pair
+//    instructions (add, subtract, fma of (re, im)): one issue slot instead of
+//    two, with the rounding of the scalar forms.
+//  * A butterfly e +- w o with w = c (1 - i T), T = tan, is u = o (1 - i T)
+//    (two scalar fma) and e +- c u (two packed fma): 4 instructions instead of
+//    8.  Each component is rounded twice instead of three times.
+//  * The inter-pass twiddles are not applied to the operands before a radix-R
+//    kernel but inside its butterflies, stage by stage, where a twiddle costs
+//    nothing beyond the table load: a radix-R pass needs R/2 pairs (c, T) per
+//    thread, one of each pair of twiddles that differ by a quarter turn.
 #pragma once
+#include <cmath>
 #include <type_traits>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -37,6 +50,22 @@ __host__ __device__ __forceinline__ C cmk(typename ElemOf<C>::type a, typename E
 }
 template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return cmk<C>(a.x + b.x, a.y + b.y); }
 template <typename C> __device__ __forceinline__ C csub(C a, C b) { return cmk<C>(a.x - b.x, a.y - b.y); }
+// e + c u for real c
+__device__ __forceinline__ double2 cfma(double c, double2 u, double2 e) {
+  return make_double2(fma(c, u.x, e.x), fma(c, u.y, e.y));
+}
+#ifdef __CUDA_ARCH__
+// the packed FP32 forms (sm_100a)
+template <> __device__ __forceinline__ float2 cadd<float2>(float2 a, float2 b) { return __fadd2_rn(a, b); }
+template <> __device__ __forceinline__ float2 csub<float2>(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+}
+__device__ __forceinline__ float2 cfma(float c, float2 u, float2 e) { return __ffma2_rn(make_float2(c, c), u, e); }
+#else
+__device__ __forceinline__ float2 cfma(float c, float2 u, float2 e) {
+  return make_float2(fmaf(c, u.x, e.x), fmaf(c, u.y, e.y));
+}
+#endif
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -107,45 +136,80 @@ __device__ __forceinline__ C tw_const(C o) {
   }
 }
 
-// ---------------------------------------------------------------------------
 // In-register DFT of R points v[0], v[S], ..., v[(R-1)S] (natural order in
-// and out), forward sign.  Radix-2 decimation in time, radix-4 and radix-3
-// leaves.
+// and out), forward sign (INV: backward).  Radix-2 decimation in time,
+// radix-4 and radix-3 leaves.
 // ---------------------------------------------------------------------------
-template <int R, int S, typename C> __device__ __forceinline__ void dft_s(C* v);
+template <int R, int S, bool INV = false, typename C> __device__ __forceinline__ void dft_s(C* v);
 
-template <int K, int R, int S, typename C>
-__device__ __forceinline__ void dit2_combine(C* v, C* tmp) {
-  if constexpr (K < R / 2) {
-    C e = v[2 * S * K];
-    C o = tw_const<K, R>(v[S + 2 * S * K]);
-    tmp[K] = cadd(e, o);
-    tmp[K + R / 2] = csub(e, o);
-    dit2_combine<K + 1, R, S>(v, tmp);
+// p = e + w o, m = e - w o with w = c (1 - i T) (INV: its conjugate), turned
+// by a further -i (INV: +i) if QUARTER
+template <bool INV, bool QUARTER, typename C>
+__device__ __forceinline__ void bfly(C e, C o, typename ElemOf<C>::type c, typename ElemOf<C>::type T, C& p, C& m) {
+  C u;
+  if constexpr (!INV && !QUARTER) u = cmk<C>(fma(T, o.y, o.x), fma(-T, o.x, o.y));
+  else if constexpr (INV && !QUARTER) u = cmk<C>(fma(-T, o.y, o.x), fma(T, o.x, o.y));
+  else if constexpr (!INV) u = cmk<C>(fma(-T, o.x, o.y), fma(-T, o.y, -o.x));
+  else u = cmk<C>(fma(-T, o.x, -o.y), fma(-T, o.y, o.x));
+  p = cfma(c, u, e);
+  m = cfma(-c, u, e);
+}
+
+// p = e -+ i o, m = e +- i o (upper signs: forward); the swapped components
+// make scalar sums the shorter form
+template <bool INV, typename C>
+__device__ __forceinline__ void bfly_quarter(C e, C o, C& p, C& m) {
+  const C a = cmk<C>(e.x + o.y, e.y - o.x), b = cmk<C>(e.x - o.y, e.y + o.x);
+  p = INV ? b : a;
+  m = INV ? a : b;
+}
+
+// butterfly K of a radix-R combine step: p, m = e +- W_R^K o, 0 <= K < R/2
+template <int K, int R, bool INV, typename C>
+__device__ __forceinline__ void bfly_const(C e, C o, C& p, C& m) {
+  using T = typename ElemOf<C>::type;
+  if constexpr (K == 0) {
+    p = cadd(e, o);
+    m = csub(e, o);
+  } else if constexpr (4 * K == R) {
+    bfly_quarter<INV>(e, o, p, m);
+  } else {
+    constexpr bool Q = 4 * K > R;
+    // angle of the twiddle after the quarter turn: 2 pi j / (4 R) in (0, pi/2)
+    constexpr int j = 4 * K - (Q ? R : 0);
+    bfly<INV, Q>(e, o, T(ct_trig(j, 4 * R, 0)), T(ct_trig(j, 4 * R, 1) / ct_trig(j, 4 * R, 0)), p, m);
   }
 }
 
-template <int K, int R, int S, typename C>
+template <int K, int R, int S, bool INV, typename C>
+__device__ __forceinline__ void dit2_combine(C* v, C* tmp) {
+  if constexpr (K < R / 2) {
+    bfly_const<K, R, INV>(v[2 * S * K], v[S + 2 * S * K], tmp[K], tmp[K + R / 2]);
+    dit2_combine<K + 1, R, S, INV>(v, tmp);
+  }
+}
+
+template <int K, int R, int S, bool INV, typename C>
 __device__ __forceinline__ void dit3_combine(C* v, C* tmp) {
   using T = typename ElemOf<C>::type;
   if constexpr (K < R / 3) {
     constexpr int M = R / 3;
     C a = v[3 * S * K];
-    C b = tw_const<K, R>(v[S + 3 * S * K]);
-    C c = tw_const<2 * K, R>(v[2 * S + 3 * S * K]);
-    // radix-3 butterfly, W3 = exp(-2 pi i/3) = (-1/2, -sqrt(3)/2)
-    constexpr T h = T(0.86602540378443864676);
+    C b = tw_const<INV ? -K : K, R>(v[S + 3 * S * K]);
+    C c = tw_const<INV ? -2 * K : 2 * K, R>(v[2 * S + 3 * S * K]);
+    // radix-3 butterfly, W3 = exp(-+2 pi i/3) = (-1/2, -+sqrt(3)/2)
+    constexpr T h = INV ? T(-0.86602540378443864676) : T(0.86602540378443864676);
     C s = cadd(b, c), d = csub(b, c);
     C m = cmk<C>(a.x - T(0.5) * s.x, a.y - T(0.5) * s.y);
-    C r = cmk<C>(h * d.y, -h * d.x);   // -i*sqrt(3)/2 * d
+    C r = cmk<C>(h * d.y, -h * d.x);   // -+i*sqrt(3)/2 * d
     tmp[K] = cadd(a, s);
     tmp[K + M] = cadd(m, r);
     tmp[K + 2 * M] = csub(m, r);
-    dit3_combine<K + 1, R, S>(v, tmp);
+    dit3_combine<K + 1, R, S, INV>(v, tmp);
   }
 }
 
-template <int R, int S, typename C>
+template <int R, int S, bool INV, typename C>
 __device__ __forceinline__ void dft_s(C* v) {
   if constexpr (R == 1) {
   } else if constexpr (R == 2) {
@@ -154,29 +218,68 @@ __device__ __forceinline__ void dft_s(C* v) {
     v[S] = csub(a, b);
   } else if constexpr (R == 4) {
     C a = v[0], b = v[S], c = v[2 * S], d = v[3 * S];
-    C t0 = cadd(a, c), t1 = csub(a, c), t2 = cadd(b, d), t3 = cmul_mi(csub(b, d));
+    C t0 = cadd(a, c), t1 = csub(a, c), t2 = cadd(b, d), t3 = csub(b, d);
     v[0] = cadd(t0, t2);
     v[2 * S] = csub(t0, t2);
-    v[S] = cadd(t1, t3);
-    v[3 * S] = csub(t1, t3);
+    bfly_quarter<INV>(t1, t3, v[S], v[3 * S]);
   } else if constexpr (R % 4 == 0 || R % 2 == 0 && R % 3 != 0) {
-    dft_s<R / 2, 2 * S>(v);
-    dft_s<R / 2, 2 * S>(v + S);
+    dft_s<R / 2, 2 * S, INV>(v);
+    dft_s<R / 2, 2 * S, INV>(v + S);
     C tmp[R];
-    dit2_combine<0, R, S>(v, tmp);
+    dit2_combine<0, R, S, INV>(v, tmp);
 #pragma unroll
     for (int k = 0; k < R; k++) v[S * k] = tmp[k];
   } else if constexpr (R % 3 == 0) {
-    dft_s<R / 3, 3 * S>(v);
-    dft_s<R / 3, 3 * S>(v + S);
-    dft_s<R / 3, 3 * S>(v + 2 * S);
+    dft_s<R / 3, 3 * S, INV>(v);
+    dft_s<R / 3, 3 * S, INV>(v + S);
+    dft_s<R / 3, 3 * S, INV>(v + 2 * S);
     C tmp[R];
-    dit3_combine<0, R, S>(v, tmp);
+    dit3_combine<0, R, S, INV>(v, tmp);
 #pragma unroll
     for (int k = 0; k < R; k++) v[S * k] = tmp[k];
   } else {
     static_assert(R % 2 == 0 || R % 3 == 0, "unsupported radix");
   }
+}
+
+// Twiddled DFT of a pass p >= 1: v[q] <- sum_r v[r] W_(NS R)^(r (k + NS q)),
+// R a power of two, natural order in and out.  Decimation in time: the
+// combine step of radix rho = 2, 4, .., R multiplies its odd half by
+// W_(NS rho)^(k + NS q'), q' < rho/2, of which q' and q' + rho/4 differ by a
+// quarter turn.  tw[row * NS] holds this thread's (c, T): row 0 for rho = 2,
+// row rho/4 + q' for rho >= 4 (q' < rho/4); see build_twiddles.
+template <int R, int NS, bool INV, typename C>
+__device__ __forceinline__ void dft_tw(C* v, const C* __restrict__ tw) {
+  static_assert(R >= 2 && (R & (R - 1)) == 0, "power-of-two radix");
+  constexpr int LOG = R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : R == 16 ? 4 : R == 32 ? 5 : 6;
+  C a[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    int j = 0;
+#pragma unroll
+    for (int b = 0; b < LOG; b++) j |= ((i >> b) & 1) << (LOG - 1 - b);
+    a[i] = v[j];
+  }
+  {
+    const C w = tw[0];
+#pragma unroll
+    for (int b = 0; b < R; b += 2) bfly<INV, false>(a[b], a[b + 1], w.x, w.y, a[b], a[b + 1]);
+  }
+#pragma unroll
+  for (int l = 2; l <= LOG; l++) {
+    const int rho = 1 << l;
+#pragma unroll
+    for (int q = 0; q < rho / 4; q++) {
+      const C w = tw[(rho / 4 + q) * NS];
+#pragma unroll
+      for (int b = q; b < R; b += rho) {
+        bfly<INV, false>(a[b], a[b + rho / 2], w.x, w.y, a[b], a[b + rho / 2]);
+        bfly<INV, true>(a[b + rho / 4], a[b + 3 * rho / 4], w.x, w.y, a[b + rho / 4], a[b + 3 * rho / 4]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R; i++) v[i] = a[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -215,17 +318,9 @@ __host__ __device__ constexpr int plan_e(int N, bool dbl) {
 __host__ __device__ constexpr int plan_ns(int N, bool dbl, int p) {
   int s = 1; for (int i = 0; i < p; i++) s *= plan_rad(N, dbl, i); return s;
 }
-// Passes p >= 1 of radix >= 16 (a multiple of 8) keep factored twiddles:
-// W^(r k) = W^(8 (r/8) k) * W^((r%8) k), rows [0..7] of W^(r0 k) then rows
-// [8 .. 8 + R/8 - 1] of W^(8 r1 k), so a thread loads 8 + R/8 twiddles
-// instead of R (radix 32: 12 instead of 32) and forms the rest with one
-// complex product each.
-__host__ __device__ constexpr bool plan_fact(int N, bool dbl, int p) {
-  return p >= 1 && plan_rad(N, dbl, p) >= 16 && plan_rad(N, dbl, p) % 8 == 0;
-}
+// (c, T) pairs of pass p >= 1: R/2 rows of NS (dft_tw)
 __host__ __device__ constexpr int plan_twsz(int N, bool dbl, int p) {
-  return plan_fact(N, dbl, p) ? (8 + plan_rad(N, dbl, p) / 8) * plan_ns(N, dbl, p)
-                              : plan_rad(N, dbl, p) * plan_ns(N, dbl, p);
+  return plan_rad(N, dbl, p) / 2 * plan_ns(N, dbl, p);
 }
 __host__ __device__ constexpr int plan_twoff(int N, bool dbl, int p) {
   int o = 0; for (int i = 1; i < p; i++) o += plan_twsz(N, dbl, i); return o;
@@ -242,7 +337,6 @@ template <typename T, int N> struct FFTPlan {
   static_assert(P * E == N, "operands per thread must divide the line");
   static constexpr int ns(int p) { return plan_ns(N, DBL, p); }
   static constexpr int twoff(int p) { return plan_twoff(N, DBL, p); }
-  static constexpr bool fact(int p) { return plan_fact(N, DBL, p); }
   static constexpr int TWSIZE = plan_twoff(N, DBL, plan_npass(N, DBL)) > 0 ? plan_twoff(N, DBL, plan_npass(N, DBL)) : 1;
 };
 
@@ -263,38 +357,23 @@ __device__ __forceinline__ void line_sync() {
 
 // Operands of butterfly set q of thread t in one Stockham pass: read from the
 // line, twiddled, transformed in registers (v[q R .. q R + R - 1]).
-template <typename C, int N, int R, int NS, int E, int P, bool FACT>
+template <typename C, int N, int R, int NS, int E, int P, bool INV = false>
 __device__ __forceinline__ void pass_butterflies(const C* line, int t, const C* __restrict__ twp, C* v) {
   constexpr int NB = E / R;
 #pragma unroll
   for (int q = 0; q < NB; q++) {
     const int j = t + q * P;
-    const int k = j % NS;
 #pragma unroll
     for (int r = 0; r < R; r++) v[q * R + r] = line[pad32(j + r * (N / R))];
-    if constexpr (FACT) {
-      C t0[8];
-#pragma unroll
-      for (int r0 = 1; r0 < 8; r0++) t0[r0] = twp[r0 * NS + k];
-#pragma unroll
-      for (int r0 = 1; r0 < 8; r0++) v[q * R + r0] = cmul(v[q * R + r0], t0[r0]);
-#pragma unroll
-      for (int r1 = 1; r1 < R / 8; r1++) {
-        const C t1 = twp[(8 + r1) * NS + k];
-        v[q * R + 8 * r1] = cmul(v[q * R + 8 * r1], t1);
-#pragma unroll
-        for (int r0 = 1; r0 < 8; r0++) v[q * R + 8 * r1 + r0] = cmul(v[q * R + 8 * r1 + r0], cmul(t1, t0[r0]));
-      }
-    } else if constexpr (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; r++) v[q * R + r] = cmul(v[q * R + r], twp[r * NS + k]);
-    }
-    dft_s<R, 1>(v + q * R);
+    if constexpr (NS > 1)
+      dft_tw<R, NS, INV>(v + q * R, twp + j % NS);
+    else
+      dft_s<R, 1, INV>(v + q * R);
   }
 }
 
 // One Stockham pass over nlines lines (rounds of LPR lines).
-template <typename C, int N, int R, int NS, int E, int P, int THREADS, bool FACT>
+template <typename C, int N, int R, int NS, int E, int P, int THREADS, bool INV = false>
 __device__ __forceinline__ void fft_pass(C* buf, int nlines, int ls, const C* __restrict__ twp) {
   constexpr int LPR = THREADS / P;
   constexpr int NB = E / R;   // butterflies per thread
@@ -306,7 +385,7 @@ __device__ __forceinline__ void fft_pass(C* buf, int nlines, int ls, const C* __
     const bool act = (lr < LPR) && (l < nlines);
     C v[E];
     C* line = buf + (size_t)l * ls;
-    if (act) pass_butterflies<C, N, R, NS, E, P, FACT>(line, t, twp, v);
+    if (act) pass_butterflies<C, N, R, NS, E, P, INV>(line, t, twp, v);
     line_sync<P>();
     if (act) {
 #pragma unroll
@@ -322,14 +401,14 @@ __device__ __forceinline__ void fft_pass(C* buf, int nlines, int ls, const C* __
   }
 }
 
-template <typename T, int N, int THREADS, int PASS>
+template <typename T, int N, int THREADS, int PASS, bool INV = false>
 __device__ __forceinline__ void fft_passes(C2<T>* buf, int nlines, int ls, const C2<T>* tw) {
   using PL = FFTPlan<T, N>;
   if constexpr (PASS < PL::NPASS) {
     constexpr int R = PL::rad(PASS);
     constexpr int NS = PL::ns(PASS);
-    fft_pass<C2<T>, N, R, NS, PL::E, PL::P, THREADS, PL::fact(PASS)>(buf, nlines, ls, tw + PL::twoff(PASS));
-    fft_passes<T, N, THREADS, PASS + 1>(buf, nlines, ls, tw);
+    fft_pass<C2<T>, N, R, NS, PL::E, PL::P, THREADS, INV>(buf, nlines, ls, tw + PL::twoff(PASS));
+    fft_passes<T, N, THREADS, PASS + 1, INV>(buf, nlines, ls, tw);
   }
 }
 
@@ -352,7 +431,7 @@ __device__ __forceinline__ void fft_lines(C2<T>* buf, int nlines, int ls, const 
 // together whatever branches fix takes.  Pass 0 has no twiddles; its output
 // goes to the line in shared memory, so the staging copy of the input (a
 // shared-memory write and read per element) disappears.
-template <typename T, int N, int THREADS, typename Begin, typename Fetch, typename Fix>
+template <typename T, int N, int THREADS, bool INV = false, typename Begin, typename Fetch, typename Fix>
 __device__ __forceinline__ void fft_pass0_load(C2<T>* buf, int nlines, int ls, Begin begin, Fetch fetch, Fix fix) {
   using C = C2<T>;
   using PL = FFTPlan<T, N>;
@@ -377,7 +456,7 @@ __device__ __forceinline__ void fft_pass0_load(C2<T>* buf, int nlines, int ls, B
 #pragma unroll
       for (int q = 0; q < NB; q++) {
         const int j = t + q * P;
-        dft_s<R, 1>(v + q * R);
+        dft_s<R, 1, INV>(v + q * R);
 #pragma unroll
         for (int r = 0; r < R; r++) line[pad32(j * R + r)] = v[q * R + r];
       }
@@ -387,14 +466,14 @@ __device__ __forceinline__ void fft_pass0_load(C2<T>* buf, int nlines, int ls, B
 
 // fft_lines with pass 0 fed by fft_pass0_load; waits for the caller's
 // cp.async twiddle copies before the passes that use them.
-template <typename T, int N, int THREADS, typename Begin, typename Fetch, typename Fix>
+template <typename T, int N, int THREADS, bool INV = false, typename Begin, typename Fetch, typename Fix>
 __device__ __forceinline__ void fft_lines_load(C2<T>* buf, int nlines, int ls, const C2<T>* tw, Begin begin,
                                                Fetch fetch, Fix fix) {
   static_assert(THREADS % FFTPlan<T, N>::P == 0, "THREADS must be a multiple of threads per line");
-  fft_pass0_load<T, N, THREADS>(buf, nlines, ls, begin, fetch, fix);
+  fft_pass0_load<T, N, THREADS, INV>(buf, nlines, ls, begin, fetch, fix);
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-  fft_passes<T, N, THREADS, 1>(buf, nlines, ls, tw);
+  fft_passes<T, N, THREADS, 1, INV>(buf, nlines, ls, tw);
   __syncthreads();
 }
 
@@ -403,7 +482,7 @@ __device__ __forceinline__ void fft_lines_load(C2<T>* buf, int nlines, int ls, c
 // r NS (r < R, natural order) of line l in vals[r] (R and NS as
 // std::integral_constant), typically as global stores, so the pass output is
 // not written to shared memory and read back.
-template <typename T, int N, int THREADS, typename Begin, typename Store>
+template <typename T, int N, int THREADS, bool INV = false, typename Begin, typename Store>
 __device__ __forceinline__ void fft_pass_last_store(const C2<T>* buf, int nlines, int ls, const C2<T>* tw,
                                                     Begin begin, Store store) {
   using C = C2<T>;
@@ -416,7 +495,7 @@ __device__ __forceinline__ void fft_pass_last_store(const C2<T>* buf, int nlines
     const int l = l0 + lr;
     if (l < nlines) {
       C v[E];
-      pass_butterflies<C, N, R, NS, E, P, PL::fact(PASS)>(buf + (size_t)l * ls, t, tw + PL::twoff(PASS), v);
+      pass_butterflies<C, N, R, NS, E, P, INV>(buf + (size_t)l * ls, t, tw + PL::twoff(PASS), v);
       const auto s = begin(l);
 #pragma unroll
       for (int q = 0; q < NB; q++) {
@@ -429,59 +508,59 @@ __device__ __forceinline__ void fft_pass_last_store(const C2<T>* buf, int nlines
   }
 }
 
-template <typename T, int N, int THREADS, int PASS, int LAST>
+template <typename T, int N, int THREADS, int PASS, int LAST, bool INV = false>
 __device__ __forceinline__ void fft_passes_until(C2<T>* buf, int nlines, int ls, const C2<T>* tw) {
   using PL = FFTPlan<T, N>;
   if constexpr (PASS < LAST) {
     constexpr int R = PL::rad(PASS);
     constexpr int NS = PL::ns(PASS);
-    fft_pass<C2<T>, N, R, NS, PL::E, PL::P, THREADS, PL::fact(PASS)>(buf, nlines, ls, tw + PL::twoff(PASS));
-    fft_passes_until<T, N, THREADS, PASS + 1, LAST>(buf, nlines, ls, tw);
+    fft_pass<C2<T>, N, R, NS, PL::E, PL::P, THREADS, INV>(buf, nlines, ls, tw + PL::twoff(PASS));
+    fft_passes_until<T, N, THREADS, PASS + 1, LAST, INV>(buf, nlines, ls, tw);
   }
 }
 
 // Whole transform with pass 0 fed by fetch and fix (fft_pass0_load) and the last pass
 // handing its outputs to store: shared memory holds only the exchanges
 // between passes.  Needs a plan of two passes or more.
-template <typename T, int N, int THREADS, typename LBegin, typename Fetch, typename Fix, typename SBegin,
-          typename Store>
+template <typename T, int N, int THREADS, bool INV = false, typename LBegin, typename Fetch, typename Fix,
+          typename SBegin, typename Store>
 __device__ __forceinline__ void fft_lines_load_store(C2<T>* buf, int nlines, int ls, const C2<T>* tw,
                                                      LBegin lbegin, Fetch fetch, Fix fix, SBegin sbegin,
                                                      Store store) {
   using PL = FFTPlan<T, N>;
   static_assert(PL::NPASS >= 2, "load and store passes must differ");
   static_assert(THREADS % PL::P == 0, "THREADS must be a multiple of threads per line");
-  fft_pass0_load<T, N, THREADS>(buf, nlines, ls, lbegin, fetch, fix);
+  fft_pass0_load<T, N, THREADS, INV>(buf, nlines, ls, lbegin, fetch, fix);
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-  fft_passes_until<T, N, THREADS, 1, PL::NPASS - 1>(buf, nlines, ls, tw);
-  fft_pass_last_store<T, N, THREADS>(buf, nlines, ls, tw, sbegin, store);
+  fft_passes_until<T, N, THREADS, 1, PL::NPASS - 1, INV>(buf, nlines, ls, tw);
+  fft_pass_last_store<T, N, THREADS, INV>(buf, nlines, ls, tw, sbegin, store);
 }
 
-// Host: build the twiddle table of FFTPlan<T,N> (pass p >= 1 table is
-// [r][k] = W_N^(r k N/(Ns R)), r < R, k < Ns; factored passes hold the rows
-// r0 = 0..7 and 8 r1, r1 = 0..R/8-1, see plan_fact).
+// Host: build the twiddle table of FFTPlan<T,N>: for every pass p >= 1 the
+// pairs (c, T) = (cos, tan) of the angle 2 pi (k + NS q') / (NS rho) of
+// dft_tw's combine steps, [row][k] with k < NS.  The angle pi/2 (rho = 2,
+// k = NS/2), whose tangent does not exist, is stored as c = 2^-40 (FP64
+// 2^-80), T = 1/c: c T = 1 exactly and the remaining c o.x is far below the
+// rounding of the sum it enters.
 template <typename T, int N>
 void build_twiddles(C2<T>* out) {
   using PL = FFTPlan<T, N>;
-  auto w = [](long m) {
-    // accurate angle: reduce m/N to [0,1) exactly in integers
-    m %= N;
-    long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)N;
-    return cmk<C2<T>>((T)cosl(ang), (T)sinl(ang));
+  auto pair = [](long num, long den) {   // angle 2 pi num / den in [0, pi)
+    if (4 * num == den) {
+      const T c = std::ldexp(T(1), sizeof(T) == 8 ? -80 : -40);
+      return cmk<C2<T>>(c, T(1) / c);
+    }
+    const long double ang = 2.0L * 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
+    return cmk<C2<T>>((T)cosl(ang), (T)(sinl(ang) / cosl(ang)));
   };
   for (int p = 1; p < PL::NPASS; p++) {
     const int R = PL::rad(p), NS = PL::ns(p), off = PL::twoff(p);
-    const long s = N / (NS * R);
-    if (PL::fact(p)) {
-      for (int k = 0; k < NS; k++) {
-        for (int r0 = 0; r0 < 8; r0++) out[off + r0 * NS + k] = w((long)r0 * k * s);
-        for (int r1 = 0; r1 < R / 8; r1++) out[off + (8 + r1) * NS + k] = w((long)8 * r1 * k * s);
+    for (int rho = 2; rho <= R; rho *= 2)
+      for (int q = 0; q < (rho == 2 ? 1 : rho / 4); q++) {
+        C2<T>* row = out + off + (rho == 2 ? 0 : rho / 4 + q) * NS;
+        for (int k = 0; k < NS; k++) row[k] = pair(k + (long)NS * q, (long)NS * rho);
       }
-    } else {
-      for (int r = 0; r < R; r++)
-        for (int k = 0; k < NS; k++) out[off + r * NS + k] = w((long)r * k * s);
-    }
   }
 }
 

@@ -122,6 +122,9 @@ __host__ __device__ __forceinline__ size_t ubi_var_elems(int nab_i, int n) {
   return (size_t)((nab_i + R - 1) / R * R) * Tiles<T>::TB_I * n;
 }
 
+// conj(v) if CJ (a backward transform made of a forward one)
+template <bool CJ, typename C> __device__ __forceinline__ C conj_if(C v) { return CJ ? cconj(v) : v; }
+
 template <int N> __device__ __forceinline__ int kwave(int i) { return i > N / 2 ? i - N : i; }
 
 __device__ __forceinline__ bool mask_ok(const Geo& g, int a, int y, int n) {
@@ -276,8 +279,9 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
     }
     return s;
   };
-  // fetch: the shifted entry (zero where masked); fix: derivative, prefilter
-  // and the conjugation of the backward transform (zero stays zero)
+  // fetch: the shifted entry (zero where masked); fix: derivative and
+  // prefilter (zero stays zero), and for the tensor-core form, which only
+  // transforms forward, the conjugation of the backward transform
   auto fetch = [&](const Col& s, int y) {
     const int ky = y > N / 2 ? N - y : y;
     C val = cmk<C>(0, 0);
@@ -295,7 +299,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
       }
     }
     if constexpr (SPL) val = cscale(s.fx * __ldg(st.spf + (N / 2 + 1) + y) * s.fz, val);
-    return cconj(val);
+    return conj_if<TCM>(val);
   };
   if constexpr (TCM) {
     tc::Work w;
@@ -308,7 +312,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
         [](C* p, int k, C v) { p[pad32(k)] = v; });
     tc::teardown<NCOL>(w);
   } else {
-    fft_lines_load<T, N, THREADS>(buf, TB, L, tw, begin, fetch, fix);
+    fft_lines_load<T, N, THREADS, true>(buf, TB, L, tw, begin, fetch, fix);
   }
   // columns a0 + l sit at ((a / TBL) n + y) TBL + a % TBL of variable v: a
   // block writes 64-byte halves of the 128-byte runs (a sequential pair of
@@ -317,7 +321,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
   C* out = ub + (size_t)v * ubi_var_elems<T>(g.nab_i, N) + (size_t)(at / R) * N * TBL + (at % R) * TB;
   for (int e = threadIdx.x; e < TB * N; e += THREADS) {
     const int y = e / TB, l = e % TB;
-    out[y * TBL + l] = cconj(buf[l * L + pad32(y)]);
+    out[y * TBL + l] = conj_if<TCM>(buf[l * L + pad32(y)]);
   }
 }
 
@@ -387,7 +391,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
         val = cmk<C>(-bk * val.y, bk * val.x);
       }
     }
-    return cconj(val);
+    return conj_if<TCM>(val);
   };
   // the last pass stores its outputs straight to uz: line l, entry z at
   // ((v n + y) nzt + z / TZ) kxn + x0 + l) TZ + z % TZ (consecutive z of a
@@ -400,7 +404,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
     static_assert(NS % TZ == 0, "last-pass stride must keep z % TZ");
     C* p = d + ((unsigned)base / TZ) * zstride + (unsigned)base % TZ;
 #pragma unroll
-    for (int r = 0; r < R; r++) p[(size_t)(r * (NS / TZ)) * zstride] = cconj(vals[r]);
+    for (int r = 0; r < R; r++) p[(size_t)(r * (NS / TZ)) * zstride] = vals[r];
   };
   if constexpr (TCM) {
     tc::Work w;
@@ -412,7 +416,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
         [&](C* d, int z, C v) { d[((unsigned)z / TZ) * zstride + (unsigned)z % TZ] = cconj(v); });
     tc::teardown<NCOL>(w);
   } else {
-    fft_lines_load_store<T, N, THREADS>(buf, nl, L, tw, begin, fetch, fix, sbegin, store);
+    fft_lines_load_store<T, N, THREADS, true>(buf, nl, L, tw, begin, fetch, fix, sbegin, store);
   }
 }
 
@@ -610,7 +614,7 @@ __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf
     const bool act = l < nlines;
     C v[E];
     if (act) {
-      pass_butterflies<C, N, R1, NS, E, P, PL::fact(1)>(buf + (size_t)l * L, t, tw + PL::twoff(1), v);
+      pass_butterflies<C, N, R1, NS, E, P>(buf + (size_t)l * L, t, tw + PL::twoff(1), v);
     } else {
 #pragma unroll
       for (int m = 0; m < E; m++) v[m] = cmk<C>(0, 0);
