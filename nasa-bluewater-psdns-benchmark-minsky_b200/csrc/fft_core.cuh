@@ -10,9 +10,9 @@
 // thread owns E/R_p butterflies of radix R_p whose operands it holds in
 // registers; the radix-R kernels are unrolled at compile time.  Between passes
 // data goes through shared memory in place: all operands are read, the block
-// synchronises, then all results are written.  Shared-memory element i of a
-// line lives at pad(i) = i + i/32, which keeps the strided writes of the first
-// pass from serialising on one bank.
+// synchronises, then all results are written.  Element i of a line lives at
+// padl(i), which keeps the strided writes of the first pass from serialising
+// on one bank.
 //
 // What bounds the transforms inside the kernels is the number of instructions
 // issued, not the FMA pipe (the x chain issued 0.59 per cycle and scheduler at
@@ -340,16 +340,43 @@ template <typename T, int N> struct FFTPlan {
   static constexpr int TWSIZE = plan_twoff(N, DBL, plan_npass(N, DBL)) > 0 ? plan_twoff(N, DBL, plan_npass(N, DBL)) : 1;
 };
 
-__host__ __device__ __forceinline__ constexpr int pad32(int i) { return i + (i >> 5); }
-template <int N> struct LineLen { static constexpr int value = N + N / 32; };
+// Shared-memory place of element i of a line: i + i/R0 for a power-of-two
+// first radix R0 (i + i/32 otherwise).  Pass 0 writes with a stride of R0
+// between threads, which then becomes R0 + 1: no two threads of a phase meet
+// on a bank (with i/32 for every plan the 16-point first passes of n = 256 and
+// 512 met two by two, the 8-point ones of FP64 n = 512 four by four).
+__host__ __device__ constexpr int pad_shift(int N, bool dbl) {
+  return is_pow2(plan_rad(N, dbl, 0)) ? ilog2c(plan_rad(N, dbl, 0)) : 5;
+}
+template <typename C, int N>
+__host__ __device__ __forceinline__ constexpr int padl(int i) {
+  return i + (i >> pad_shift(N, sizeof(C) == 16));
+}
+// elements from one line to the next: N and its padding, rounded up to
+// residue M modulo 16 (FP32) or 8 (FP64), the banks of one phase.  4 (8 for
+// eight threads a line) keeps the lines that share a phase apart in every
+// pass; see the kernels for other residues.
+__host__ __device__ constexpr int line_stride(int N, bool dbl, int M) {
+  const int mod = dbl ? 8 : 16;
+  int l = N + (N >> pad_shift(N, dbl));
+  while (l % mod != M % mod) l++;
+  return l;
+}
+template <typename T, int N> struct LS {
+  static constexpr bool DBL = sizeof(T) == 8;
+  static constexpr int value = line_stride(N, DBL, !DBL && N / plan_e(N, DBL) == 8 ? 8 : 4);
+};
 
-// Barrier among the threads that share a line.  When a line lives inside one
-// warp (P divides 32) a warp barrier suffices; otherwise the whole block
-// synchronises.
+// Barrier among the threads that share a line.  A warp barrier where lines
+// live inside warps; where a line is P / 32 whole warps, the named barrier of
+// the line's group (1 + its index in the block, at most 15 groups), so that the
+// lines of a block do not wait for one another.
 template <int P>
 __device__ __forceinline__ void line_sync() {
   if constexpr (P <= 32 && (32 % P) == 0) {
     __syncwarp();
+  } else if constexpr (P % 32 == 0) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / P), "n"(P) : "memory");
   } else {
     __syncthreads();
   }
@@ -364,7 +391,7 @@ __device__ __forceinline__ void pass_butterflies(const C* line, int t, const C* 
   for (int q = 0; q < NB; q++) {
     const int j = t + q * P;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[q * R + r] = line[pad32(j + r * (N / R))];
+    for (int r = 0; r < R; r++) v[q * R + r] = line[padl<C, N>(j + r * (N / R))];
     if constexpr (NS > 1)
       dft_tw<R, NS, INV>(v + q * R, twp + j % NS);
     else
@@ -394,7 +421,7 @@ __device__ __forceinline__ void fft_pass(C* buf, int nlines, int ls, const C* __
         const int k = j % NS;
         const int base = (j / NS) * NS * R + k;
 #pragma unroll
-        for (int r = 0; r < R; r++) line[pad32(base + r * NS)] = v[q * R + r];
+        for (int r = 0; r < R; r++) line[padl<C, N>(base + r * NS)] = v[q * R + r];
       }
     }
     line_sync<P>();
@@ -413,7 +440,7 @@ __device__ __forceinline__ void fft_passes(C2<T>* buf, int nlines, int ls, const
 }
 
 // Forward FFT of nlines lines in shared memory (line l at buf + l*ls,
-// element i at pad32(i)); tw = shared twiddle table of FFTPlan<T,N>.
+// element i at padl(i)); tw = shared twiddle table of FFTPlan<T,N>.
 // Must be called by all THREADS threads of the block (contains barriers).
 template <typename T, int N, int THREADS>
 __device__ __forceinline__ void fft_lines(C2<T>* buf, int nlines, int ls, const C2<T>* tw) {
@@ -458,7 +485,7 @@ __device__ __forceinline__ void fft_pass0_load(C2<T>* buf, int nlines, int ls, B
         const int j = t + q * P;
         dft_s<R, 1, INV>(v + q * R);
 #pragma unroll
-        for (int r = 0; r < R; r++) line[pad32(j * R + r)] = v[q * R + r];
+        for (int r = 0; r < R; r++) line[padl<C, N>(j * R + r)] = v[q * R + r];
       }
     }
   }

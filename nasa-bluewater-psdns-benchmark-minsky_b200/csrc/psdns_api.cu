@@ -329,13 +329,14 @@ static int upload_tables(Ctx& c) {
 template <typename T, int N, int NC> struct Impl {
   using C = C2<T>;
   using TL = Tiles<T>;
-  static constexpr int L = LS<N>::value;
+  static constexpr int L = LS<T, N>::value;
   static constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
-  static size_t sm1() { return TWB + sizeof(C) * TL::TB_I * L; }
+  static size_t sm1() { return K1Launch<T, N>::SMEM; }
   static size_t sm2() { return TWB + sizeof(C) * TL::XT2 * L; }
   static size_t sm3() { return K3Launch<T, N, NC>::SMEM; }
   static size_t sm4() { return K4Launch<T, N>::SMEM; }
   static size_t sm5() { return TWB + sizeof(C) * (4 + NC) * TL::TB_F * L; }
+  static size_t sm1tc() { return TWB + sizeof(C) * TL::TB_I * L + kTcTail; }
   static size_t sm2tc() { return TWB + sizeof(C) * kTcXT2 * L + kTcTail; }
   static size_t sm4tc() { return K4LaunchX<T, N, kTcXT4, true>::SMEM + kTcTail; }
 
@@ -347,7 +348,7 @@ template <typename T, int N, int NC> struct Impl {
   static int setup() {
     if constexpr (kTc) {
       CK(cudaFuncSetAttribute(k_yinv<T, N, false, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sm1() + kTcTail)));
+                              (int)sm1tc()));
       CK(cudaFuncSetAttribute(k_zinv<T, N, NC, false, true, kTcXT2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm2tc()));
       CK(cudaFuncSetAttribute(k_xchain<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -558,7 +559,7 @@ template <typename T, int N, int NC> struct Impl {
     const int s = kstep - 1;
     prof_mark(c, s, 0, 0);
     k_yinv<T, N, false, NC, true><<<dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), K1Launch<T, N>::THREADS,
-                                    sm1() + kTcTail, c.stream>>>(g, st, u, ub, tw, ta);
+                                    sm1tc(), c.stream>>>(g, st, u, ub, tw, ta);
     prof_mark(c, s, 0, 1);
     prof_mark(c, s, 1, 0);
     k_zinv<T, N, NC, false, true, kTcXT2><<<dim3(N, (kxn + kTcXT2 - 1) / kTcXT2, 3 + 3 * NC),

@@ -169,11 +169,15 @@ struct Launch {
   static_assert(THREADS % P == 0, "threads per line must divide the block");
 };
 
-template <int N> struct LS { static constexpr int value = N + N / 32 + 4; };
-
 // K1 and K4: one warp per line at n = 1024 FP32
 template <typename T, int N>
-struct K1Launch : Launch<T, N, Tiles<T>::TB_I, 1024> {};
+struct K1Launch : Launch<T, N, Tiles<T>::TB_I, 1024> {
+  // its transposed store reads TB_I lines at two y a phase: a line stride of 2
+  // modulo the banks keeps them apart (not the tensor-core form's, n = 1024)
+  static constexpr bool DBL = sizeof(T) == 8;
+  static constexpr int L = Launch<T, N, Tiles<T>::TB_I, 1024>::P >= 16 ? line_stride(N, DBL, 2) : LS<T, N>::value;
+  static constexpr size_t SMEM = sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)Tiles<T>::TB_I * L);
+};
 // K4 with XT x lines per block: three fields of every x line at once
 // (register-fed form, phase 1 of k_zfwd), or two (tensor-core form)
 template <typename T, int N, int XT, bool TCM = false>
@@ -186,7 +190,7 @@ struct K4LaunchX : Launch<T, N, (TCM ? 2 : 3) * XT * Tiles<T>::YT4, 1024> {
   static constexpr int MINB_F = 65536 / (TH * 112) < 1 ? 1 : (65536 / (TH * 112) > 8 ? 8 : 65536 / (TH * 112));
   static constexpr int MINB = TCM ? 2 : MINB_F;
   static constexpr size_t SMEM =
-      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)NF * XT * Tiles<T>::YT4 * LS<N>::value);
+      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)NF * XT * Tiles<T>::YT4 * LS<T, N>::value);
 };
 template <typename T, int N>
 struct K4Launch : K4LaunchX<T, N, k4_xt(sizeof(T) == 8, N)> {};
@@ -254,7 +258,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
   using C = C2<T>;
   constexpr int TB = Tiles<T>::TB_I;
   constexpr int THREADS = K1Launch<T, N>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = TCM ? LS<T, N>::value : K1Launch<T, N>::L;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* buf = tw + FFTPlan<T, N>::TWSIZE;
@@ -309,7 +313,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
     tc::fft1024<THREADS>(
         TB, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * L * sizeof(C)), begin,
         [&](const Col& s, int y) { return fix(s, y, fetch(s, y)); }, line,
-        [](C* p, int k, C v) { p[pad32(k)] = v; });
+        [](C* p, int k, C v) { p[padl<C, N>(k)] = v; });
     tc::teardown<NCOL>(w);
   } else {
     fft_lines_load<T, N, THREADS, true>(buf, TB, L, tw, begin, fetch, fix);
@@ -321,7 +325,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
   C* out = ub + (size_t)v * ubi_var_elems<T>(g.nab_i, N) + (size_t)(at / R) * N * TBL + (at % R) * TB;
   for (int e = threadIdx.x; e < TB * N; e += THREADS) {
     const int y = e / TB, l = e % TB;
-    out[y * TBL + l] = conj_if<TCM>(buf[l * L + pad32(y)]);
+    out[y * TBL + l] = conj_if<TCM>(buf[l * L + padl<C, N>(y)]);
   }
 }
 
@@ -352,7 +356,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
   constexpr int XT = XTO > 0 ? XTO : Tiles<T>::XT2, TZ = Tiles<T>::TZ;
   static_assert(!TCM || XT >= 4, "an operand tile overlays four lines");
   constexpr int THREADS = Launch<T, N, XT>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* buf = tw + FFTPlan<T, N>::TWSIZE;
@@ -441,8 +445,8 @@ __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int
   for (int b = 0; b < nbuf; b++)
   for (int x = x0; x < kxn; x += xs) {
     const C* line = buf + (b * NPAIR + p) * L;
-    const C Y = line[pad32(x)];
-    const C Yn = line[pad32(x == 0 ? 0 : N - x)];
+    const C Y = line[padl<C, N>(x)];
+    const C Yn = line[padl<C, N>(x == 0 ? 0 : N - x)];
     const C A = cmk<C>((Y.x + Yn.x) * half_factor, (Y.y - Yn.y) * half_factor);
     const C B = cmk<C>((Y.y + Yn.y) * half_factor, (Yn.x - Y.x) * half_factor);
     C* dst = uz + ((((size_t)(slot0 + b) * N + y) * g.nzt + zt) * kxn + x) * TZ + 2 * p;
@@ -492,10 +496,10 @@ __device__ __forceinline__ void xchain_pack(const Geo& g, const C2<T>* __restric
         const C a = A[v][i], b = B[v][i];
         C* line = bufU + (v * NPAIR + p) * L;
         if (x == 0) {
-          line[pad32(0)] = cmk<C>(a.x, -b.x);
+          line[padl<C, N>(0)] = cmk<C>(a.x, -b.x);
         } else {
-          line[pad32(x)] = cmk<C>(a.x - b.y, -(a.y + b.x));
-          line[pad32(N - x)] = cmk<C>(a.x + b.y, -(b.x - a.y));
+          line[padl<C, N>(x)] = cmk<C>(a.x - b.y, -(a.y + b.x));
+          line[padl<C, N>(N - x)] = cmk<C>(a.x + b.y, -(b.x - a.y));
         }
       }
     }
@@ -585,7 +589,7 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
         dft_s<R0, 1>(w);
         const int j = t + q * P;
 #pragma unroll
-        for (int r = 0; r < R0; r++) line[pad32(j * R0 + r)] = w[r];
+        for (int r = 0; r < R0; r++) line[padl<C, N>(j * R0 + r)] = w[r];
       }
     }
   }
@@ -655,12 +659,12 @@ struct K3Launch {
   static_assert(THREADS % P == 0, "threads per line must divide the block");
   // twiddles + 5 product buffers (6 input buffers with a scalar) of TZ/2 lines
   static constexpr size_t SMEM =
-      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)(NC ? 6 : 5) * NPAIR * LS<N>::value);
+      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)(NC ? 6 : 5) * NPAIR * LS<T, N>::value);
   // tensor-core form: the line buffers rounded up to whole tiles of four
   // lines (the operands overlay them), then the tail
   static constexpr int LINES_TC = ((NC ? 6 : 5) * NPAIR + 3) / 4 * 4;
   static constexpr size_t SMEM_TC =
-      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)LINES_TC * LS<N>::value) + kTcTail;
+      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)LINES_TC * LS<T, N>::value) + kTcTail;
 };
 
 template <typename T, int N, int NC = 0, bool TCM = false>
@@ -675,7 +679,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
   constexpr int NVIN = 3 + 3 * NC;
   constexpr int THREADS = K3Launch<T, N, NC>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* bufU = tw + FFTPlan<T, N>::TWSIZE;
@@ -707,7 +711,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
     // zero the band kx in [kxn, n-kxn] (includes the Nyquist column)
     for (int e = threadIdx.x; e < NVIN * NPAIR * N; e += THREADS) {
       const int k = e % N;
-      if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + pad32(k)] = cmk<C>(0, 0);
+      if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
     }
     xchain_pack<T, N, 3, THREADS>(g, uz, 0, y, zt, bufU, L);
     if constexpr (NC > 0) xchain_pack<T, N, 3, THREADS>(g, uz, 3, y, zt, bufU + 3 * NPAIR * L, L);
@@ -723,7 +727,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   double vm = 0.0;
   const double xn = (double)b11 * N, yn = (double)b22 * N, zn = (double)b33 * N;
   for (int e = threadIdx.x; e < NPAIR * N; e += THREADS) {
-    const int i = (e / N) * L + pad32(e % N);
+    const int i = (e / N) * L + padl<C, N>(e % N);
     const C U = bufU[i], V = bufV[i], W = bufW[i];
     if constexpr (NC > 0) {
       C* bufGZ = bufF + NPAIR * L;
@@ -781,7 +785,7 @@ __device__ __forceinline__ void zfwd_load(const Geo& g, const C2<T>* __restrict_
     const unsigned cnt = (NLC > 0 ? NLC : nl) * N;
     for (unsigned e = threadIdx.x; e < cnt; e += blockDim.x) {
       const unsigned zt = e / w, rem = e % w, l = rem / TZ, zz = rem % TZ;
-      cp_async_elem(b + l * L + pad32(zt * TZ + zz), src + ((size_t)zt * g.kxn + l) * TZ + zz);
+      cp_async_elem(b + l * L + padl<C2<T>, N>(zt * TZ + zz), src + ((size_t)zt * g.kxn + l) * TZ + zz);
     }
   };
   for (int yy = 0; yy < ny; yy++) {
@@ -825,7 +829,7 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
       if (a >= csr[j]) { lx = j; c0 = csr[j]; c1 = csr[j + 1]; }
     const int kc = (c1 - c0 - 1) / 2, ia = a - c0;
     const int x = x0 + lx, z = ia <= kc ? ia : ia + N - (2 * kc + 1), l = yy * nl + lx;
-    const int i = l * L + pad32(z);
+    const int i = l * L + padl<C, N>(z);
     C out;
     if constexpr (MODE == 0) {          // i kx P1 + i b33 kz P5   (s1 = P1, s0 = P5)
       const T kx = T(x), bk3 = b33 * T(kwave<N>(z));
@@ -864,7 +868,7 @@ __device__ __forceinline__ void zfwd_fused(const Geo& g, const C2<T>* __restrict
   using PL = FFTPlan<T, N>;
   static_assert(Tiles<T>::YT4 == 1, "one y row per block");
   static_assert(PL::NPASS >= 2, "load and store passes must differ");
-  constexpr int TZ = Tiles<T>::TZ, TB = Tiles<T>::TBL_F, L = LS<N>::value;
+  constexpr int TZ = Tiles<T>::TZ, TB = Tiles<T>::TBL_F, L = LS<T, N>::value;
   constexpr size_t zstride = (size_t)kxn_of(N) * TZ;   // g.kxn, as a constant
   const size_t var = ubf_var_elems<T>(g.nab_f, N);
   // uz field `slot` of x line x0 + xl at row y: entry z at (z / TZ) zstride + z % TZ
@@ -892,11 +896,11 @@ __device__ __forceinline__ void zfwd_fused(const Geo& g, const C2<T>* __restrict
       C out = v[r];
       if (s.mode == 0) {
         const T kx = T(s.x), bk3 = b33 * T(kwave<N>(z));
-        const C p5 = s.p5[pad32(z)];
+        const C p5 = s.p5[padl<C, N>(z)];
         out = cmk<C>(-kx * v[r].y - bk3 * p5.y, kx * v[r].x + bk3 * p5.x);
       } else if (s.mode == 1) {
         const T bk1 = b11 * T(s.x), kz = T(kwave<N>(z));
-        const C p5 = s.p5[pad32(z)];
+        const C p5 = s.p5[padl<C, N>(z)];
         out = cmk<C>(-bk1 * p5.y - kz * v[r].y, bk1 * p5.x + kz * v[r].x);
       }
       const int a = s.c0 + (z <= s.kc ? z : z - N + 2 * s.kc + 1);
@@ -939,7 +943,7 @@ k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>*
   constexpr int XT = XTO > 0 ? XTO : k4_xt(sizeof(T) == 8, N), YT = Tiles<T>::YT4, NLT = XT * YT;
   static_assert(!TCM || NLT >= 4, "an operand tile overlays four lines of s0 or s1");
   constexpr int THREADS = K4LaunchX<T, N, XT, TCM>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* s0 = tw + FFTPlan<T, N>::TWSIZE;
@@ -1054,7 +1058,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   constexpr int TB = Tiles<T>::TB_F;
   constexpr int NVF = 4 + NC;
   constexpr int THREADS = K5Launch<T, N, NC>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* buf = tw + FFTPlan<T, N>::TWSIZE;   // [4][TB] lines
@@ -1068,7 +1072,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
     const C* src = ub + (size_t)v * ubf_var_elems<T>(g.nab_f, N) + (size_t)(at / R) * N * TBL + (at % R) * TB;
     for (int e = threadIdx.x; e < TB * N; e += THREADS) {
       const int y = e / TB, l = e % TB;
-      cp_async_elem(buf + (v * TB + l) * L + pad32(y), src + y * TBL + l);
+      cp_async_elem(buf + (v * TB + l) * L + padl<C, N>(y), src + y * TBL + l);
     }
   }
   const size_t vs = (size_t)g.xz_tot * N;
@@ -1117,7 +1121,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
     const int x = __ldg(g.ax + a), z = __ldg(g.az + a);
     const int iky = kwave<N>(y), ikz = kwave<N>(z);
     const T kx = T(x), ky = T(iky), kz = T(ikz);
-    const int i = pad32(y);
+    const int i = padl<C, N>(y);
     const C V1 = buf[(0 * TB + l) * L + i], V2 = buf[(1 * TB + l) * L + i];
     const C V3 = buf[(2 * TB + l) * L + i], V4 = buf[(3 * TB + l) * L + i];
     // wavespace_vel.f:165-169
@@ -1276,7 +1280,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
   using V4 = typename V4T<T>::type;
   constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
   constexpr int THREADS = Launch<T, N, 2 * TZ>::THREADS;
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* bufU = tw + FFTPlan<T, N>::TWSIZE;
@@ -1292,7 +1296,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
   } else {
     for (int e = threadIdx.x; e < 3 * NPAIR * N; e += THREADS) {
       const int k = e % N;
-      if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + pad32(k)] = cmk<C>(0, 0);
+      if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
     }
     xchain_pack<T, N, 3, THREADS>(g, uz, 0, y, zt, bufU, L);
     cp_async_wait_all();
@@ -1302,7 +1306,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
   // buffer = conj(a + i b): line z = 2p is re, line 2p+1 is -im
   for (int e = threadIdx.x; e < TZ * N; e += THREADS) {
     const int zz = e / N, x = e % N, p = zz / 2;
-    const int i = p * L + pad32(x);
+    const int i = p * L + padl<C, N>(x);
     const C U = bufU[i], V = bufU[NPAIR * L + i], W = bufU[2 * NPAIR * L + i];
     V4 c;
     if (zz & 1) { c.x = -U.y; c.y = -V.y; c.z = -W.y; } else { c.x = U.x; c.y = V.x; c.z = W.x; }
@@ -1320,7 +1324,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
 template <typename T, int N>
 struct KMomLaunch : Launch<T, N, 2 * (Tiles<T>::TZ / 2)> {
   static constexpr size_t SMEM =
-      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)2 * (Tiles<T>::TZ / 2) * LS<N>::value);
+      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)2 * (Tiles<T>::TZ / 2) * LS<T, N>::value);
 };
 
 template <typename T, int N>
@@ -1330,7 +1334,7 @@ k_xmoments(Geo g, const C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, 
   constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
   constexpr int THREADS = KMomLaunch<T, N>::THREADS;
   static_assert(THREADS % 32 == 0, "the reduction uses whole warps");
-  constexpr int L = LS<N>::value;
+  constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* bufU = tw + FFTPlan<T, N>::TWSIZE;
@@ -1339,7 +1343,7 @@ k_xmoments(Geo g, const C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, 
   const int zt = blockIdx.x, y = blockIdx.y, kxn = g.kxn;
   for (int e = threadIdx.x; e < 2 * NPAIR * N; e += THREADS) {
     const int k = e % N;
-    if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + pad32(k)] = cmk<C>(0, 0);
+    if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
   }
   xchain_pack<T, N, 2, THREADS>(g, uz, 0, y, zt, bufU, L);
   cp_async_wait_all();
@@ -1353,7 +1357,7 @@ k_xmoments(Geo g, const C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, 
     const int zz = e / N, x = e % N, p = zz / 2;
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-      const C z = bufU[(f * NPAIR + p) * L + pad32(x)];
+      const C z = bufU[(f * NPAIR + p) * L + padl<C, N>(x)];
       const double v = (zz & 1) ? -(double)z.y : (double)z.x, sq = v * v;
       s[8 * f + 0] += v;
       s[8 * f + 1] += sq;

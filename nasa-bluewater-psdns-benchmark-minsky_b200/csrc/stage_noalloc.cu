@@ -98,8 +98,6 @@ static Plan plan_for(const Geometry& g) {
   return p;
 }
 
-template <int N> struct Ls { static constexpr int value = N + N / 32 + 4; };
-
 template <typename T, int N>
 static int run(const psdns_params* prm, int kstep, const double* gsh, double dt, C2<T>* u, C2<T>* un,
                double* velmax_out, cudaStream_t st) {
@@ -187,12 +185,12 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   C* uz = (C*)(base + pl.uz);
   const C* twd = (const C*)(base + pl.tw);
   unsigned long long* vmx = (unsigned long long*)(base + pl.velmax);
-  constexpr int L = Ls<N>::value;
+  constexpr int L = LS<T, N>::value;
   constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
   const int kxn = g.kxn;
   {
     constexpr int TH = K1Launch<T, N>::THREADS;
-    k_yinv<T, N><<<dim3(k1_blocks<T>(geo.nab_i), 3), TH, TWB + sizeof(C) * TL::TB_I * L, st>>>(geo, stb, u, ub, twd);
+    k_yinv<T, N><<<dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st>>>(geo, stb, u, ub, twd);
   }
   {
     constexpr int TH = Launch<T, N, TL::XT2>::THREADS;

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256) k_dft_lines(const float2* __restrict__ in
                                                    long long nlines, const float2* __restrict__ tw_g,
                                                    const uint4* __restrict__ btab, const float2* __restrict__ tw2,
                                                    unsigned* err) {
-  constexpr int N = 1024, NL = 8, THREADS = 256, L = LS<N>::value;
+  constexpr int N = 1024, NL = 8, THREADS = 256, L = LS<float, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* tws = reinterpret_cast<float2*>(smem_raw);
   float2* buf = tws + FFTPlan<float, N>::TWSIZE;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) k_dft_lines(const float2* __restrict__ in
   const int nl = (int)(nlines - l0 < NL ? nlines - l0 : NL);
   for (int e = threadIdx.x; e < nl * N; e += THREADS) {
     const int l = e / N, i = e % N;
-    buf[l * L + pad32(i)] = in[(l0 + l) * N + i];
+    buf[l * L + padl<float2, 1024>(i)] = in[(l0 + l) * N + i];
   }
   if constexpr (MODE == 0) {
     load_twiddles<float, N>(tws, tw_g);
@@ -148,12 +148,12 @@ __global__ void __launch_bounds__(256) k_dft_lines(const float2* __restrict__ in
   __syncthreads();
   for (int e = threadIdx.x; e < nl * N; e += THREADS) {
     const int l = e / N, i = e % N;
-    out[(l0 + l) * N + i] = buf[l * L + pad32(i)];
+    out[(l0 + l) * N + i] = buf[l * L + padl<float2, 1024>(i)];
   }
 }
 
 constexpr size_t dft_smem() {
-  return sizeof(float2) * (FFTPlan<float, 1024>::TWSIZE + 8 * LS<1024>::value) + kBBytes + 16;
+  return sizeof(float2) * (FFTPlan<float, 1024>::TWSIZE + 8 * LS<float, 1024>::value) + kBBytes + 16;
 }
 
 }  // namespace tc

@@ -356,7 +356,7 @@ __device__ __forceinline__ void fft1024(int nlines, Work& w, unsigned char* tile
 }
 
 // fft1024 on lines held in shared memory, line l at buf + l ls, element i
-// at pad32(i) (the layout of fft_lines), in place.  The operand tiles
+// at padl(i) (the layout of fft_lines), in place.  The operand tiles
 // overlay lines 4t .. 4t + 3 (ls * 8 * 4 >= 32 KB bytes, 16-byte aligned):
 // the storage of every line up to the next multiple of four is
 // overwritten.  Ends with a barrier.
@@ -365,7 +365,7 @@ __device__ __forceinline__ void fft1024_lines(float2* buf, int nlines, int ls, W
   auto line = [&](int l) { return buf + (size_t)l * ls; };
   fft1024<THREADS>(
       nlines, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * ls * sizeof(float2)), line,
-      [](const float2* p, int i) { return p[pad32(i)]; }, line, [](float2* p, int k, float2 v) { p[pad32(k)] = v; });
+      [](const float2* p, int i) { return p[padl<float2, 1024>(i)]; }, line, [](float2* p, int k, float2 v) { p[padl<float2, 1024>(k)] = v; });
   __syncthreads();
 }
 
