@@ -657,6 +657,8 @@ struct K3Launch {
   static constexpr int WP = 32 / gcd_c(32, P) * P;   // lcm(32, P): whole warps and whole lines
   static constexpr int THREADS = round_up(want, WP) > 1024 ? 1024 : round_up(want, WP);
   static_assert(THREADS % P == 0, "threads per line must divide the block");
+  // registers sized for twenty warps per SM (about 100 a thread)
+  static constexpr int MINB = 640 / THREADS < 2 ? 2 : (640 / THREADS > 10 ? 10 : 640 / THREADS);
   // twiddles + 5 product buffers (6 input buffers with a scalar) of TZ/2 lines
   static constexpr size_t SMEM =
       sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)(NC ? 6 : 5) * NPAIR * LS<T, N>::value);
@@ -667,8 +669,26 @@ struct K3Launch {
       sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)LINES_TC * LS<T, N>::value) + kTcTail;
 };
 
+// One grid point's part of velmax (realspace_vel.f:105-114) for the two real
+// lines of a pair: vm <- max(vm, xn |u| + yn |v| + zn |w|) in FP64.  For an
+// FP32 state the sum is first taken in FP32, whose relative error (all terms
+// positive, five roundings) is below 4e-7: a point whose FP32 sum is below
+// (1 - 1e-6) vm cannot raise vm and skips its six conversions to FP64.
+template <typename C>
+__device__ __forceinline__ void velmax_point(C U, C V, C W, double xn, double yn, double zn, double& vm) {
+  if constexpr (sizeof(C) == 8) {
+    const float fx = (float)xn, fy = (float)yn, fz = (float)zn;
+    const float ea = fmaf(fx, fabsf(U.x), fmaf(fy, fabsf(V.x), fz * fabsf(W.x)));
+    const float eb = fmaf(fx, fabsf(U.y), fmaf(fy, fabsf(V.y), fz * fabsf(W.y)));
+    if (fmaxf(ea, eb) < __double2float_rd(vm) * 0.999999f) return;
+  }
+  const double va = xn * fabs((double)U.x) + yn * fabs((double)V.x) + zn * fabs((double)W.x);
+  const double vb = xn * fabs((double)U.y) + yn * fabs((double)V.y) + zn * fabs((double)W.y);
+  vm = fmax(vm, fmax(va, vb));
+}
+
 template <typename T, int N, int NC = 0, bool TCM = false>
-__global__ void __launch_bounds__(K3Launch<T, N, NC>::THREADS, TCM ? 1 : 2)
+__global__ void __launch_bounds__(K3Launch<T, N, NC>::THREADS, TCM ? 1 : K3Launch<T, N, NC>::MINB)
 k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T b22, T b33,
          unsigned long long* velmax_bits, int want_velmax, T cb1 = T(0), T cb2 = T(0), T cb3 = T(0),
          TcArgs tca = TcArgs()) {
@@ -724,7 +744,11 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   // realspace_vel.f:105-114, in place: slot 0 = b11 u^2 - bv2, 1 = uv,
   // 2 = b33 w^2 - bv2, 3 = vw (is1), 4 = uw (is2); velmax at stage 1.  With
   // a scalar, slot 5 = its advection term (buffer 5 held d/dz theta).
+  // this thread's velmax starts from what the blocks before have found, so that
+  // few points are summed in FP64
   double vm = 0.0;
+  if (want_velmax) vm = __longlong_as_double((long long)__ldcg(velmax_bits));
+  const double vm0 = vm;
   const double xn = (double)b11 * N, yn = (double)b22 * N, zn = (double)b33 * N;
   for (int e = threadIdx.x; e < NPAIR * N; e += THREADS) {
     const int i = (e / N) * L + padl<C, N>(e % N);
@@ -736,11 +760,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
       const T sb = (-U.y) * (cb1 - GX.y) + (-V.y) * (cb2 - GY.y) + (-W.y) * (cb3 - GZ.y);
       bufGZ[i] = cmk<C>(sa, sb);
     }
-    if (want_velmax) {
-      double va = xn * fabs((double)U.x) + yn * fabs((double)V.x) + zn * fabs((double)W.x);
-      double vb = xn * fabs((double)U.y) + yn * fabs((double)V.y) + zn * fabs((double)W.y);
-      vm = fmax(vm, fmax(va, vb));
-    }
+    if (want_velmax) velmax_point(U, V, W, xn, yn, zn, vm);
     // the sign of b cancels in the mixed products
     bufF[i] = cmk<C>(U.x * W.x, U.y * W.y);
     bufE[i] = cmk<C>(V.x * W.x, V.y * W.y);
@@ -750,8 +770,8 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
     bufV[i] = cmk<C>(ua * va, ub * vb);
     bufU[i] = cmk<C>(b11 * ua * ua - bva, b11 * ub * ub - bvb);
   }
-  if (want_velmax) {
-    // block max through warp shuffles then one atomic per warp
+  if (want_velmax && __any_sync(0xffffffffu, vm > vm0)) {
+    // warp maximum through shuffles, then one atomic
     for (int o = 16; o > 0; o >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, o));
     if ((threadIdx.x & 31) == 0) atomic_max_pos<T>(velmax_bits, vm);
   }
