@@ -57,7 +57,7 @@ static int ens_alloc_class(EnsClass& e) {
   e.st_elems = up((size_t)3 * e.g.xz_tot * n);
   const size_t ubi = dbl ? ubi_var_elems<double>(e.nab_i, n) : ubi_var_elems<float>(e.nab_i, n);
   e.ub_elems = up(std::max((size_t)3 * ubi, (size_t)4 * (dbl ? ubf_var_elems<double>(e.nab_f, n) : ubf_var_elems<float>(e.nab_f, n))));
-  e.uz_elems = up((size_t)5 * n * n * e.g.kxn);
+  e.uz_elems = up((size_t)5 * n * (dbl ? uz_slab<double>(n) : uz_slab<float>(n)));
   e.tab_bytes = dbl ? TabLayout<double>(n).total : TabLayout<float>(n).total;
   const size_t nb = e.nb;
   size_t freeb = 0, totb = 0;
@@ -402,16 +402,14 @@ int psdns_gpu_ensemble_tuning(void* ens, int32_t cap, double* out, int32_t* ncla
   *nclasses = (int32_t)E->cls.size();
   for (size_t i = 0; i < E->cls.size() && (int32_t)i < cap && out; i++) {
     const EnsClass& e = *E->cls[i];
-    const int xt2 = e.prec == PSDNS_PREC_FP64 ? Tiles<double>::XT2 : Tiles<float>::XT2;
-    const int xt4 = k4_xt(e.prec == PSDNS_PREC_FP64, e.n);
-    const int m[3][2] = {{1, 1}, {1, 2}, {2, 1}};   // tile factor of variant 0, 1, 2: num/den
+    const int m[3] = {1, 2, 4};   // tile factor of variant 0, 1, 2
     double* r = out + 8 * i;
     r[0] = e.n;
     r[1] = e.nb;
     r[2] = e.tuned ? 1 : 0;
     r[3] = e.sub > 0 ? e.sub : e.nb;
-    r[4] = xt2 * m[e.k2v][0] / m[e.k2v][1];
-    r[5] = xt4 * m[e.k4v][0] / m[e.k4v][1];
+    r[4] = e.tile_lines * m[e.k2v];
+    r[5] = e.tile_lines * m[e.k4v];
     r[6] = e.default_ms;
     r[7] = e.best_ms;
   }

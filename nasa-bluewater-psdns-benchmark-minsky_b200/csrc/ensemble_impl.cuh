@@ -40,12 +40,14 @@ struct EnsClass {
   // fastest is kept for the captured graph.
   int sub = 0;
   bool tuned = false;
-  // the tuner also chooses the FFT tiles of K2 and K4 (x lines per block:
-  // variant 0 = Tiles<T>, 1 = half, 2 = double; boxes of n <= 128 only).
+  // the tuner also chooses the FFT tiles of K2 and K4 (panels of tile_lines x
+  // lines per block: variant 0 = ZLaunch's default, 1 = twice, 2 = four times as
+  // many; boxes of n <= 128 only).
   // Phases: 0 sub-batch size, 1 K2 tile, 2 K4 tile; every candidate runs
   // two real steps and keeps the faster (the first also loads its kernels).
   int k2v = 0, k4v = 0;
   bool tile_tune = false;   // n <= 128
+  int tile_lines = 0;
   int phase = 0, trial = 0, rep = 0;
   struct Cand { int sub, k2v, k4v; };
   std::vector<Cand> cands;
@@ -102,21 +104,24 @@ template <typename T, int N> struct EnsImpl {
   // tile variants of K2 and K4 are instantiated for small boxes only
   static constexpr bool kTiles = N <= 128;
 
-  // K2 / K4 with XT x lines per block (0: the default tile)
-  template <int XT>
+  // K2 / K4 with F times the default panels per block (panels of a box that
+  // has fewer are left out)
+  template <int F> static constexpr int ppb() { return F == 1 ? 0 : F * ZLaunch<T, N, 0>::PPB; }
+  template <int F>
   static void k2(EnsClass& e, const Geo& g, const C* ub, C* uz, const C* tw, const StageTables<T>& st, int nb) {
-    if constexpr (XT == 0 || kTiles) {
-      constexpr int X = XT > 0 ? XT : TL::XT2;
-      k_zinv<T, N, 0, false, false, XT><<<dim3(N, (e.g.kxn + X - 1) / X, 3 * nb), Launch<T, N, X>::THREADS,
-                                          I::TWB + sizeof(C) * X * I::L, e.stream>>>(g, ub, uz, tw, st.b11, st.b33);
+    if constexpr (F == 1 || kTiles) {
+      using Z = ZLaunch<T, N, ppb<F>()>;
+      k_zinv<T, N, 0, false, false, ppb<F>()><<<dim3(N, Z::TILES, 3 * nb), Z::THREADS, Z::SMEM2, e.stream>>>(
+          g, ub, uz, tw, st.b11, st.b33);
     }
   }
-  template <int XT>
+  template <int F>
   static void k4(EnsClass& e, const Geo& g, const C* uz, C* ub, const C* tw, const StageTables<T>& st, int nb) {
-    if constexpr (XT == 0 || kTiles) {
-      constexpr int X = XT > 0 ? XT : k4_xt(sizeof(T) == 8, N);
-      k_zfwd<T, N, 0, false, XT><<<dim3(N / TL::YT4, (e.g.kxn + X - 1) / X, nb), K4LaunchX<T, N, X>::THREADS,
-                                   K4LaunchX<T, N, X>::SMEM, e.stream>>>(g, uz, ub, tw, st.b11, st.b33);
+    if constexpr (F == 1 || kTiles) {
+      using Z = ZLaunch<T, N, ppb<F>()>;
+      const int tiles = N * Z::TILES * nb;
+      k_zfwd<T, N, 0, false, ppb<F>()><<<std::min(tiles, 148 * Z::MINB4), Z::THREADS, Z::SMEM4, e.stream>>>(
+          g, uz, ub, tw, tiles, st.b11, st.b33);
     }
   }
 
@@ -128,19 +133,18 @@ template <typename T, int N> struct EnsImpl {
     C* u = (C*)e.d_u + (size_t)b0 * e.st_elems;
     C* ub = (C*)e.d_ub + (size_t)b0 * e.ub_elems;
     C* uz = (C*)e.d_uz + (size_t)b0 * e.uz_elems;
-    const int kxn = e.g.kxn;
     k_yinv<T, N><<<dim3(k1_blocks<T>(e.nab_i), 3, nb), K1Launch<T, N>::THREADS, I::sm1(), e.stream>>>(g, st, u, ub, tw);
     switch (kTiles ? e.k2v : 0) {
-      case 1: k2<TL::XT2 / 2>(e, g, ub, uz, tw, st, nb); break;
-      case 2: k2<TL::XT2 * 2>(e, g, ub, uz, tw, st, nb); break;
-      default: k2<0>(e, g, ub, uz, tw, st, nb);
+      case 1: k2<2>(e, g, ub, uz, tw, st, nb); break;
+      case 2: k2<4>(e, g, ub, uz, tw, st, nb); break;
+      default: k2<1>(e, g, ub, uz, tw, st, nb);
     }
     k_xchain<T, N><<<dim3(e.nzt, N, nb), K3Launch<T, N, 0>::THREADS, I::sm3(), e.stream>>>(
         g, uz, tw, st.b11, st.b22, st.b33, e.d_velmax + b0, kstep == 1 ? 1 : 0);
     switch (kTiles ? e.k4v : 0) {
-      case 1: k4<k4_xt(sizeof(T) == 8, N) / 2>(e, g, uz, ub, tw, st, nb); break;
-      case 2: k4<k4_xt(sizeof(T) == 8, N) * 2>(e, g, uz, ub, tw, st, nb); break;
-      default: k4<0>(e, g, uz, ub, tw, st, nb);
+      case 1: k4<2>(e, g, uz, ub, tw, st, nb); break;
+      case 2: k4<4>(e, g, uz, ub, tw, st, nb); break;
+      default: k4<1>(e, g, uz, ub, tw, st, nb);
     }
     CK(cudaGetLastError());
     return 0;
@@ -161,14 +165,26 @@ template <typename T, int N> struct EnsImpl {
     return 0;
   }
 
+  template <int F> static int set_smem() {
+    using Z = ZLaunch<T, N, ppb<F>()>;
+    CK(cudaFuncSetAttribute(k_zinv<T, N, 0, false, false, ppb<F>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)Z::SMEM2));
+    CK(cudaFuncSetAttribute(k_zfwd<T, N, 0, false, ppb<F>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)Z::SMEM4));
+    return 0;
+  }
+
   static int setup(EnsClass& e) {
-    if (I::setup()) return 1;
+    if (I::setup() || set_smem<1>()) return 1;
+    if constexpr (kTiles)
+      if (set_smem<2>() || set_smem<4>()) return 1;
     Ctx tmp;
     if (I::twiddles(tmp)) return 1;
     e.d_tw = tmp.d_tw;
     e.stage_a = &EnsImpl::stage_a;
     e.stage_b = &EnsImpl::stage_b;
     e.tile_tune = kTiles;
+    e.tile_lines = ZLaunch<T, N, 0>::LINES;
     return 0;
   }
 };

@@ -504,37 +504,6 @@ __device__ __forceinline__ void fft_lines_load(C2<T>* buf, int nlines, int ls, c
   __syncthreads();
 }
 
-// The last pass of the plan with its outputs handed to the caller:
-// store(s, base, vals, R, NS) with s = begin(l) receives elements base +
-// r NS (r < R, natural order) of line l in vals[r] (R and NS as
-// std::integral_constant), typically as global stores, so the pass output is
-// not written to shared memory and read back.
-template <typename T, int N, int THREADS, bool INV = false, typename Begin, typename Store>
-__device__ __forceinline__ void fft_pass_last_store(const C2<T>* buf, int nlines, int ls, const C2<T>* tw,
-                                                    Begin begin, Store store) {
-  using C = C2<T>;
-  using PL = FFTPlan<T, N>;
-  constexpr int PASS = PL::NPASS - 1;
-  constexpr int R = PL::rad(PASS), NS = PL::ns(PASS), E = PL::E, P = PL::P;
-  constexpr int LPR = THREADS / P, NB = E / R;
-  const int lr = threadIdx.x / P, t = threadIdx.x % P;
-  for (int l0 = 0; l0 < nlines; l0 += LPR) {
-    const int l = l0 + lr;
-    if (l < nlines) {
-      C v[E];
-      pass_butterflies<C, N, R, NS, E, P, INV>(buf + (size_t)l * ls, t, tw + PL::twoff(PASS), v);
-      const auto s = begin(l);
-#pragma unroll
-      for (int q = 0; q < NB; q++) {
-        const int j = t + q * P;
-        const int k = j % NS;
-        store(s, (j / NS) * NS * R + k, v + q * R, std::integral_constant<int, R>(),
-              std::integral_constant<int, NS>());
-      }
-    }
-  }
-}
-
 template <typename T, int N, int THREADS, int PASS, int LAST, bool INV = false>
 __device__ __forceinline__ void fft_passes_until(C2<T>* buf, int nlines, int ls, const C2<T>* tw) {
   using PL = FFTPlan<T, N>;
@@ -546,22 +515,136 @@ __device__ __forceinline__ void fft_passes_until(C2<T>* buf, int nlines, int ls,
   }
 }
 
-// Whole transform with pass 0 fed by fetch and fix (fft_pass0_load) and the last pass
-// handing its outputs to store: shared memory holds only the exchanges
-// between passes.  Needs a plan of two passes or more.
-template <typename T, int N, int THREADS, bool INV = false, typename LBegin, typename Fetch, typename Fix,
-          typename SBegin, typename Store>
-__device__ __forceinline__ void fft_lines_load_store(C2<T>* buf, int nlines, int ls, const C2<T>* tw,
-                                                     LBegin lbegin, Fetch fetch, Fix fix, SBegin sbegin,
-                                                     Store store) {
+// ---------------------------------------------------------------------------
+// Panels: PW lines of N points interleaved in rows of 16-byte slots, the
+// layout of the z-pencils in global memory and, unchanged, of the z transforms
+// in shared memory.  Row rho holds the entries z = rho ZS .. of every line (ZS =
+// 2 entries of an FP32 line make a slot, 1 of an FP64 line); line x sits in
+// slot x ^ sw(rho).  A panel is contiguous in global memory (64 KB at n =
+// 1024), so a block copies it whole, and the x chain, which takes one slot of
+// every line, reads and writes whole rows (128 bytes in FP32).  The rotation of
+// the slots by sw(rho) spreads consecutive z of one line over all banks.
+//
+// A line is transformed in place, in its own slots: natural order (nat) at
+// the ends, and between passes the order i ^ ((i / R0) & M) (xch), which makes
+// the strided writes of a pass conflict-free like the padding of padl.  Both
+// are linear over bitwise xor for N = 2^k, so an address is a thread's own part
+// xor a constant, and the constant's bits above the permuted ones go into the
+// instruction's immediate offset.
+// ---------------------------------------------------------------------------
+template <typename T, int N> struct Panel {
+  using C = C2<T>;
+  using PL = FFTPlan<T, N>;
+  static constexpr bool DBL = sizeof(T) == 8, POW2 = is_pow2(N);
+  static constexpr int ZS = DBL ? 1 : 2, PW = DBL ? 4 : 8;
+  static constexpr int ROW = PW * ZS;            // complex elements of a row
+  static constexpr int ELEMS = N * PW;           // of a panel
+  static constexpr unsigned BYTES = ELEMS * sizeof(C);
+  static constexpr unsigned LOW = DBL ? 511 : 1023;   // bytes that the orders permute within
+  static constexpr int S = POW2 ? ilog2c(PL::rad(0)) : 0;
+  static constexpr unsigned M = !POW2 ? 0 : (PL::rad(0) < (DBL ? 8 : 16) ? PL::rad(0) : (DBL ? 8 : 16)) - 1;
+  static_assert(N % ZS == 0 && BYTES % 1024 == 0, "panels keep the alignment that xor addressing needs");
+  __host__ __device__ static constexpr unsigned sw(unsigned rho) { return DBL ? (rho >> 1) & 3 : rho & 7; }
+  // byte offset of element i of line 0 (line x: xor 16 x)
+  template <bool XCH> __host__ __device__ static constexpr unsigned off(unsigned i) {
+    if (XCH) i ^= (i >> S) & M;
+    const unsigned rho = i / ZS;
+    return rho * (ROW * sizeof(C)) + sw(rho) * 16 + (i % ZS) * sizeof(C);
+  }
+  // element a + B of the line at byte offset o (panel offset + 16 x); the bits
+  // of a and B are disjoint for N = 2^k
+  template <bool XCH, unsigned B> __device__ __forceinline__ static C& at(unsigned char* smem, unsigned oa, unsigned o, unsigned a) {
+    if constexpr (POW2) {
+      constexpr unsigned c = off<XCH>(B);
+      return *reinterpret_cast<C*>(smem + (oa ^ (c & LOW)) + (c & ~LOW));
+    } else {
+      return *reinterpret_cast<C*>(smem + (o & ~127u) + (off<XCH>(a + B) ^ (o & 127)));
+    }
+  }
+};
+
+template <typename T, int N, bool XCH, int R, int STEP, int r = 0>
+__device__ __forceinline__ void panel_read(unsigned char* smem, unsigned oa, unsigned o, unsigned a, C2<T>* v) {
+  if constexpr (r < R) {
+    v[r] = Panel<T, N>::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a);
+    panel_read<T, N, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
+  }
+}
+template <typename T, int N, bool XCH, int R, int STEP, int r = 0>
+__device__ __forceinline__ void panel_write(unsigned char* smem, unsigned oa, unsigned o, unsigned a, const C2<T>* v) {
+  if constexpr (r < R) {
+    Panel<T, N>::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a) = v[r];
+    panel_write<T, N, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
+  }
+}
+
+// elements t + q P + r (N / R) of a line, natural order (r < R, q < E / R)
+template <typename T, int N, int R>
+__device__ __forceinline__ void panel_load(unsigned char* smem, unsigned o, int t, C2<T>* v) {
+  using PA = Panel<T, N>;
+  using PL = FFTPlan<T, N>;
+#pragma unroll
+  for (int q = 0; q < PL::E / R; q++) {
+    const unsigned a = t + q * PL::P;
+    panel_read<T, N, false, R, N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
+  }
+}
+template <typename T, int N, int R>
+__device__ __forceinline__ void panel_store(unsigned char* smem, unsigned o, int t, const C2<T>* v) {
+  using PA = Panel<T, N>;
+  using PL = FFTPlan<T, N>;
+#pragma unroll
+  for (int q = 0; q < PL::E / R; q++) {
+    const unsigned a = t + q * PL::P;
+    panel_write<T, N, false, R, N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
+  }
+}
+
+// Transform of one line by its group of P threads, exchanging through the
+// line's own slots.  v: the operands of pass 0 (element t + q P + r (N / R0) in
+// v[q R0 + r]) in, the outputs of the last pass (element t + q P + r NS in
+// v[q R + r]) out; afterwards every slot of the line has been read.  Called by
+// whole warps.
+template <typename T, int N, bool INV>
+__device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t, const C2<T>* tw, C2<T>* v) {
+  using PA = Panel<T, N>;
   using PL = FFTPlan<T, N>;
   static_assert(PL::NPASS >= 2, "load and store passes must differ");
-  static_assert(THREADS % PL::P == 0, "THREADS must be a multiple of threads per line");
-  fft_pass0_load<T, N, THREADS, INV>(buf, nlines, ls, lbegin, fetch, fix);
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
-  fft_passes_until<T, N, THREADS, 1, PL::NPASS - 1, INV>(buf, nlines, ls, tw);
-  fft_pass_last_store<T, N, THREADS, INV>(buf, nlines, ls, tw, sbegin, store);
+  constexpr int E = PL::E, P = PL::P, R0 = PL::rad(0);
+#pragma unroll
+  for (int q = 0; q < E / R0; q++) dft_s<R0, 1, INV>(v + q * R0);
+#pragma unroll
+  for (int q = 0; q < E / R0; q++) {
+    const unsigned a = (t + q * P) * R0;
+    panel_write<T, N, true, R0, 1>(smem, o ^ PA::template off<true>(a), o, a, v + q * R0);
+  }
+  line_sync<P>();
+  if constexpr (PL::NPASS == 3) {
+    constexpr int R = PL::rad(1), NS = PL::ns(1);
+#pragma unroll
+    for (int q = 0; q < E / R; q++) {
+      const unsigned a = t + q * P;
+      panel_read<T, N, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+    }
+    line_sync<P>();
+#pragma unroll
+    for (int q = 0; q < E / R; q++) {
+      const int j = t + q * P;
+      dft_tw<R, NS, INV>(v + q * R, tw + PL::twoff(1) + j % NS);
+      const unsigned a = (j / NS) * NS * R + j % NS;
+      panel_write<T, N, true, R, NS>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+    }
+    line_sync<P>();
+  }
+  constexpr int LAST = PL::NPASS - 1, R = PL::rad(LAST), NS = PL::ns(LAST);
+#pragma unroll
+  for (int q = 0; q < E / R; q++) {
+    const unsigned a = t + q * P;
+    panel_read<T, N, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+  }
+  line_sync<P>();
+#pragma unroll
+  for (int q = 0; q < E / R; q++) dft_tw<R, NS, INV>(v + q * R, tw + PL::twoff(LAST) + (t + q * P) % NS);
 }
 
 // Host: build the twiddle table of FFTPlan<T,N>: for every pass p >= 1 the

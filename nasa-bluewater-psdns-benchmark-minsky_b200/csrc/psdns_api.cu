@@ -332,13 +332,19 @@ template <typename T, int N, int NC> struct Impl {
   static constexpr int L = LS<T, N>::value;
   static constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
   static size_t sm1() { return K1Launch<T, N>::SMEM; }
-  static size_t sm2() { return TWB + sizeof(C) * TL::XT2 * L; }
+  using ZL = ZLaunch<T, N, 0>;
+  static size_t sm2() { return ZL::SMEM2; }
   static size_t sm3() { return K3Launch<T, N, NC>::SMEM; }
-  static size_t sm4() { return K4Launch<T, N>::SMEM; }
+  static size_t sm4() { return ZL::SMEM4; }
   static size_t sm5() { return TWB + sizeof(C) * (4 + NC) * TL::TB_F * L; }
   static size_t sm1tc() { return TWB + sizeof(C) * TL::TB_I * L + kTcTail; }
   static size_t sm2tc() { return TWB + sizeof(C) * kTcXT2 * L + kTcTail; }
-  static size_t sm4tc() { return K4LaunchX<T, N, kTcXT4, true>::SMEM + kTcTail; }
+  static size_t sm4tc() { return TWB + sizeof(C) * 2 * kTcXT4 * L + kTcTail; }
+  // K2: a block per tile of panels, y row and field (nf fields over all boxes);
+  // K4: its tiles, and a block for each as far as they stay resident
+  static dim3 k2_grid(int nf) { return dim3(N, ZL::TILES, nf); }
+  static int k4_tiles(int boxes) { return N * ZL::TILES * boxes; }
+  static int k4_grid(int tiles) { return std::min(tiles, 148 * ZL::MINB4); }
 
   // the tensor-core form (FP32 state at n = 1024): the same kernels with
   // their 1-D transforms on the tensor cores, and a shared-memory tail
@@ -349,11 +355,11 @@ template <typename T, int N, int NC> struct Impl {
     if constexpr (kTc) {
       CK(cudaFuncSetAttribute(k_yinv<T, N, false, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm1tc()));
-      CK(cudaFuncSetAttribute(k_zinv<T, N, NC, false, true, kTcXT2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      CK(cudaFuncSetAttribute(k_zinv<T, N, NC, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm2tc()));
       CK(cudaFuncSetAttribute(k_xchain<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)K3Launch<T, N, NC>::SMEM_TC));
-      CK(cudaFuncSetAttribute(k_zfwd<T, N, NC, true, kTcXT4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      CK(cudaFuncSetAttribute(k_zfwd<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm4tc()));
       CK(cudaFuncSetAttribute(k_yfwd<T, N, 1, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(sm5() + kTcTail)));
@@ -399,7 +405,7 @@ template <typename T, int N, int NC> struct Impl {
     prof_mark(c, 0, 5, 0);
     k_yinv<T, N, true><<<dim3(k1_blocks<T>(c.nab_i), 3), K1Launch<T, N>::THREADS, sm1(), c.stream>>>(g, st, (const C*)c.d_u,
                                                                                                ub, tw);
-    k_zinv<T, N><<<dim3(N, (kxn + TL::XT2 - 1) / TL::XT2, 3), Launch<T, N, TL::XT2>::THREADS, sm2(), c.stream>>>(
+    k_zinv<T, N><<<k2_grid(3), ZL::THREADS, sm2(), c.stream>>>(
         g, ub, uz, tw);
     using V4 = typename V4T<T>::type;
     k_xspline<T, N><<<dim3(c.nzt, N), Launch<T, N, 2 * TL::TZ>::THREADS, smxs(), c.stream>>>(g, uz, (V4*)c.d_bs, tw);
@@ -434,7 +440,7 @@ template <typename T, int N, int NC> struct Impl {
     const int kxn = c.g.kxn;
     k_yinv<T, N><<<dim3(c.nab_i, 3), K1Launch<T, N>::THREADS, sm1(), c.stream>>>(
         g, st, (const C*)(which == PSDNS_FIELD_U ? c.d_u : c.d_un), ub, tw);
-    k_zinv<T, N, 0, true><<<dim3(N, (kxn + TL::XT2 - 1) / TL::XT2, 2), Launch<T, N, TL::XT2>::THREADS, sm2(),
+    k_zinv<T, N, 0, true><<<k2_grid(2), ZL::THREADS, sm2(),
                            c.stream>>>(g, ub, uz, tw, st.b11, st.b33);
     // the transposed copy in ub is consumed: its space holds the partial sums
     double* partial = (double*)c.d_ub;
@@ -517,9 +523,8 @@ template <typename T, int N, int NC> struct Impl {
       prof_mark(c, s, 0, 1);
     }
     {
-      constexpr int TH = Launch<T, N, TL::XT2>::THREADS;
       prof_mark(c, s, 1, 0);
-      k_zinv<T, N, NC><<<dim3(N, (kxn + TL::XT2 - 1) / TL::XT2, 3 + 3 * NC), TH, sm2(), c.stream>>>(
+      k_zinv<T, N, NC><<<k2_grid(3 + 3 * NC), ZL::THREADS, sm2(), c.stream>>>(
           g, ub, uz, tw, st.b11, st.b33);
       prof_mark(c, s, 1, 1);
     }
@@ -534,11 +539,9 @@ template <typename T, int N, int NC> struct Impl {
       prof_mark(c, s, 2, 1);
     }
     {
-      constexpr int TH = K4Launch<T, N>::THREADS;
       prof_mark(c, s, 3, 0);
-      constexpr int XT4 = k4_xt(sizeof(T) == 8, N);
-      k_zfwd<T, N, NC><<<dim3(N / TL::YT4, (kxn + XT4 - 1) / XT4), TH, sm4(), c.stream>>>(g, uz, ub, tw,
-                                                                                                   st.b11, st.b33);
+      const int tiles = k4_tiles(1);
+      k_zfwd<T, N, NC><<<k4_grid(tiles), ZL::THREADS, sm4(), c.stream>>>(g, uz, ub, tw, tiles, st.b11, st.b33);
       prof_mark(c, s, 3, 1);
     }
     CK(cudaGetLastError());
@@ -562,7 +565,7 @@ template <typename T, int N, int NC> struct Impl {
                                     sm1tc(), c.stream>>>(g, st, u, ub, tw, ta);
     prof_mark(c, s, 0, 1);
     prof_mark(c, s, 1, 0);
-    k_zinv<T, N, NC, false, true, kTcXT2><<<dim3(N, (kxn + kTcXT2 - 1) / kTcXT2, 3 + 3 * NC),
+    k_zinv<T, N, NC, false, true><<<dim3(N, (kxn + kTcXT2 - 1) / kTcXT2, 3 + 3 * NC),
                                             Launch<T, N, kTcXT2>::THREADS, sm2tc(), c.stream>>>(
         g, ub, uz, tw, st.b11, st.b33, ta);
     prof_mark(c, s, 1, 1);
@@ -574,9 +577,8 @@ template <typename T, int N, int NC> struct Impl {
                                            cb2, cb3, ta);
     prof_mark(c, s, 2, 1);
     prof_mark(c, s, 3, 0);
-    k_zfwd<T, N, NC, true, kTcXT4><<<dim3(N / TL::YT4, (kxn + kTcXT4 - 1) / kTcXT4),
-                                     K4LaunchX<T, N, kTcXT4, true>::THREADS, sm4tc(), c.stream>>>(g, uz, ub, tw, st.b11,
-                                                                                          st.b33, ta);
+    k_zfwd<T, N, NC, true><<<dim3(N, (kxn + kTcXT4 - 1) / kTcXT4), Launch<T, N, 2 * kTcXT4, 1024>::THREADS, sm4tc(),
+                             c.stream>>>(g, uz, ub, tw, 0, st.b11, st.b33, ta);
     prof_mark(c, s, 3, 1);
     CK(cudaGetLastError());
     return 0;
@@ -1278,7 +1280,7 @@ int psdns_gpu_init(const psdns_params* p, void** out) {
   // (TB_F blocks); uz: 5 + nc slots (3 + 3 nc inputs, 5 + nc outputs)
   const size_t ubi = dbl ? ubi_var_elems<double>(c->nab_i, n) : ubi_var_elems<float>(c->nab_i, n);
   c->ub_elems = std::max((size_t)(3 + 2 * c->nc) * ubi, (size_t)(4 + c->nc) * (dbl ? ubf_var_elems<double>(c->nab_f, n) : ubf_var_elems<float>(c->nab_f, n)));
-  c->uz_elems = (size_t)(5 + c->nc) * n * n * c->g.kxn;
+  c->uz_elems = (size_t)(5 + c->nc) * n * (dbl ? uz_slab<double>(n) : uz_slab<float>(n));
   c->st_elems = (size_t)c->nv * c->g.xz_tot * n;
   c->rng.init(p->seed_input);
   c->dt0 = p->dt;

@@ -4,8 +4,8 @@
 //   u, un  [v][a][y]                 y-cylinders, the reference's uy(ny,num_al,v)
 //   ub     [v][a/TB][y][a%TB]         cylinder data with y and a swapped in
 //                                    blocks of TB columns (TB_I inverse, TB_F forward)
-//   uz     [v][y][z/TZ][x][z%TZ]      z-pencils for x < kxn, blocked in z so that an
-//                                    x-line tile of TZ lines is one contiguous block
+//   uz     [v][y][x/PW] panels        z-pencils for x < kxn (rounded up to panels of PW
+//                                    lines): Panel of fft_core.cuh, rows of one z slot
 // Per stage:
 //   K1 k_yinv   : phase shift + mask (phshift.f:71-135), y backward FFT
 //                 (kxcomm1_clean.f:118), transposed store into ub
@@ -47,6 +47,23 @@ __host__ __device__ constexpr int kxn_of(int n) {
   return m + 1 < n / 2 ? m + 1 : n / 2;
 }
 
+// x lines of the z-pencils: kxn rounded up to whole panels
+template <typename T>
+__host__ __device__ constexpr int kxp_of(int n) {
+  constexpr int PW = Panel<T, 1024>::PW;
+  return (kxn_of(n) + PW - 1) / PW * PW;
+}
+// elements of one y plane of one z-pencil field
+template <typename T>
+__host__ __device__ constexpr size_t uz_slab(int n) { return (size_t)kxp_of<T>(n) * n; }
+// element of (x, z) in its plane
+template <typename T, int N>
+__device__ __forceinline__ size_t uz_at(int x, int z) {
+  using PA = Panel<T, N>;
+  return (size_t)((unsigned)x / PA::PW) * PA::ELEMS +
+         ((PA::template off<false>(z) ^ (((unsigned)x % PA::PW) * 16)) / sizeof(C2<T>));
+}
+
 template <typename T> struct StageTables {
   const C2<T>* sx;   // [n/2+1] shift factors of this stage
   const C2<T>* sy;   // [n]
@@ -84,28 +101,20 @@ template <typename T> struct StageTables {
 };
 
 // per-precision tile sizes: TB_I = columns per K1 block (64 B runs in ub
-// for K2), TB_F = columns per K5 block, TZ = z lines per K3 tile (32 B
-// runs), XT2 = x lines per K2 block (K4's: k4_xt), YT4 = y rows per K4 block.
-// Eight lines per block keep two to three blocks resident per SM, so that
+// for K2), TB_F = columns per K5 block, TZ = z lines per K3 tile
+// (whole rows of the z-pencil panels).
+// Eight lines per K1 block keep two to three blocks resident per SM, so that
 // one block's copies overlap another's transforms; sixteen-line blocks (one
-// per SM) measured slower for K1 and K4.  The z transforms run smaller
-// blocks in FP32: K2 four lines (XT2 = 4) and K4 four (two x lines of two
-// fields), 4-9% faster at 512^3 and 1024^3 than eight and eight; sixteen-line
-// K2 blocks were 30% slower.
+// per SM) measured slower.
 // The inverse ub layout is blocked by TBL_I = 2 TB_I columns (128 B runs for
 // K2's reads), filled by pairs of K1 blocks.
 template <typename T> struct Tiles;
 template <> struct Tiles<float> {
-  static constexpr int TB_I = 8, TBL_I = 16, TB_F = 4, TBL_F = 8, TZ = 4, XT2 = 4, YT4 = 1;
+  static constexpr int TB_I = 8, TBL_I = 16, TB_F = 4, TBL_F = 8, TZ = 4;
 };
 template <> struct Tiles<double> {
-  static constexpr int TB_I = 4, TBL_I = 8, TB_F = 2, TBL_F = 4, TZ = 2, XT2 = 4, YT4 = 1;
+  static constexpr int TB_I = 4, TBL_I = 8, TB_F = 2, TBL_F = 4, TZ = 2;
 };
-
-// x lines per K4 block by box size (dbl: FP64 state).  FP32: four from
-// 512^3 up (1024^3: 11.44 ms against 11.77 with two), two below (256^3:
-// 0.148 ms against 0.150)
-__host__ __device__ constexpr int k4_xt(bool dbl, int n) { return dbl ? 2 : (n >= 512 ? 4 : 2); }
 
 // elements of one variable of the forward ub layout [a/TBL_F][y][a%TBL_F]
 // (K4 writes 64-byte runs; K5 blocks of TB_F columns read halves)
@@ -178,22 +187,35 @@ struct K1Launch : Launch<T, N, Tiles<T>::TB_I, 1024> {
   static constexpr int L = Launch<T, N, Tiles<T>::TB_I, 1024>::P >= 16 ? line_stride(N, DBL, 2) : LS<T, N>::value;
   static constexpr size_t SMEM = sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)Tiles<T>::TB_I * L);
 };
-// K4 with XT x lines per block: three fields of every x line at once
-// (register-fed form, phase 1 of k_zfwd), or two (tensor-core form)
-template <typename T, int N, int XT, bool TCM = false>
-struct K4LaunchX : Launch<T, N, (TCM ? 2 : 3) * XT * Tiles<T>::YT4, 1024> {
-  static constexpr int NF = TCM ? 2 : 3;
-  // resident blocks the registers are sized for: about 112 registers a
-  // thread in the register-fed form (its last pass holds a line's operands
-  // and the store addresses), one to eight blocks
-  static constexpr int TH = Launch<T, N, NF * XT * Tiles<T>::YT4, 1024>::THREADS;
-  static constexpr int MINB_F = 65536 / (TH * 112) < 1 ? 1 : (65536 / (TH * 112) > 8 ? 8 : 65536 / (TH * 112));
-  static constexpr int MINB = TCM ? 2 : MINB_F;
-  static constexpr size_t SMEM =
-      sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)NF * XT * Tiles<T>::YT4 * LS<T, N>::value);
+// Shared memory of an SM that its blocks can use, and the warps per SM that
+// the z transforms size their registers for
+constexpr size_t kSmemSM = 227 * 1024;
+constexpr int resident_blocks(size_t smem, int threads, int warps) {
+  const int a = (int)(kSmemSM / (smem + 1024)), b = warps * 32 / threads, m = a < b ? a : b;
+  return m < 1 ? 1 : (m > 16 ? 16 : m);
+}
+
+// K2 and K4: PPB panels per block (0: one, or what fills a warp), a group of P
+// threads per line
+template <typename T, int N, int PPB_>
+struct ZLaunch {
+  using PA = Panel<T, N>;
+  static constexpr int P = FFTPlan<T, N>::P;
+  static constexpr int DEF = PA::PW * P >= 32 ? 1 : 32 / (PA::PW * P);
+  static constexpr int PPB = PPB_ > 0 ? PPB_ : DEF;
+  static constexpr int LINES = PPB * PA::PW, THREADS = LINES * P;
+  static_assert(THREADS % 32 == 0 && THREADS <= 1024, "whole warps");
+  static constexpr int NPAN = kxp_of<T>(N) / PA::PW;            // panels of a plane
+  static constexpr int TILES = (NPAN + PPB - 1) / PPB;          // blocks a plane
+  static constexpr size_t TWB = sizeof(C2<T>) * FFTPlan<T, N>::TWSIZE;
+  static constexpr unsigned BUF = PPB * PA::BYTES;
+  // K2: one field's panels; sixteen warps per SM (128 registers)
+  static constexpr size_t SMEM2 = BUF + TWB;
+  static constexpr int MINB2 = resident_blocks(SMEM2, THREADS, 16);
+  // K4: three buffers
+  static constexpr size_t SMEM4 = 3 * (size_t)BUF + TWB;
+  static constexpr int MINB4 = resident_blocks(SMEM4, THREADS, 16);
 };
-template <typename T, int N>
-struct K4Launch : K4LaunchX<T, N, k4_xt(sizeof(T) == 8, N)> {};
 
 // K5 holds one CTA per SM (its (4 + nc) * TB_F lines fill shared memory), so
 // it runs every line of a block at once
@@ -335,50 +357,50 @@ __host__ __device__ __forceinline__ int k1_blocks(int nab_i) { return nab_i; }
 
 // ---------------------------------------------------------------------------
 // K2: cylinder unpack (zero fill) + z backward FFT, store to uz
-// grid (n, ceil(kxn/XT2), 3)
+// grid (n, tiles of panels, fields)
 // ---------------------------------------------------------------------------
-// XTO > 0: XTO x lines per block instead of Tiles<T>::XT2 (a tile variant
-// of the ensemble autotuner; every line is transformed the same way)
-// The FP32 velocity form's registers are sized for five resident blocks
-// (102 a thread at 128 threads): 1024^3 5.65 -> 5.33 ms against three; six
-// blocks (85, small spills) 6.01 ms.
-template <typename T, int N, int NC = 0, bool GRAD = false, bool TCM = false, int XTO = 0>
-__global__ void __launch_bounds__(Launch<T, N, (XTO > 0 ? XTO : Tiles<T>::XT2)>::THREADS,
-                                  TCM ? 2 : (sizeof(T) == 4 && NC == 0 && !GRAD ? 5 : 3))
+// One block transforms PPB panels of one field at one y (tensor-core form:
+// kTcXT2 lines).  Pass 0 takes its operands straight from ub (a warp's
+// consecutive z are consecutive cylinder columns), the lines exchange in place
+// in the panel, and the finished panel goes to uz as one bulk copy: the
+// stores of 8 bytes a lane that filled 32-byte pieces before took most of the
+// kernel's L1 cycles.  PPBO > 0: that many panels per block (a tile variant of
+// the ensemble autotuner).
+template <typename T, int N, int NC = 0, bool GRAD = false, bool TCM = false, int PPBO = 0>
+__global__ void __launch_bounds__(TCM ? Launch<T, N, kTcXT2>::THREADS : ZLaunch<T, N, PPBO>::THREADS,
+                                  TCM ? 2 : ZLaunch<T, N, PPBO>::MINB2)
 k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11 = T(1),
        T b33 = T(1), TcArgs tca = TcArgs()) {
-  // GRAD (grid.z = 2): uz slot 0 = i b11 kx u, slot 1 = i b33 kz w, the
+  // GRAD (two fields): uz slot 0 = i b11 kx u, slot 1 = i b33 kz w, the
   // gradients whose moments vgmomt.f takes (itransform.f:222-230)
-  // NC = 1 (grid.z = 6): uz slot 3 = y gradient of the scalar (ub 4), slot
+  // NC = 1 (six fields): uz slot 3 = y gradient of the scalar (ub 4), slot
   // 4 = i b11 kx theta and slot 5 = i b33 kz theta (both from ub 3),
   // itransform.f:188-198
   using C = C2<T>;
-  constexpr int XT = XTO > 0 ? XTO : Tiles<T>::XT2, TZ = Tiles<T>::TZ;
-  static_assert(!TCM || XT >= 4, "an operand tile overlays four lines");
-  constexpr int THREADS = Launch<T, N, XT>::THREADS;
-  constexpr int L = LS<T, N>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* buf = tw + FFTPlan<T, N>::TWSIZE;
+  using PL = FFTPlan<T, N>;
+  using ZL = ZLaunch<T, N, PPBO>;
+  using PA = Panel<T, N>;
+  constexpr int XT = TCM ? kTcXT2 : ZL::LINES;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  C* tw = reinterpret_cast<C*>(smem_raw + (TCM ? 0 : ZL::BUF));
   load_twiddles<T, N>(tw, tw_g);
-  // grid (n, ceil(kxn / XT2), (3 + 3 nc) * boxes)
+  // grid (n, lines / XT, fields * boxes)
   constexpr int NVZ = GRAD ? 2 : 3 + 3 * NC;
   const int y = blockIdx.x, x0 = blockIdx.y * XT, v = blockIdx.z % NVZ, box = blockIdx.z / NVZ;
   ub += box * g.bbox;
   uz += box * g.zbox;
-  const int x1 = min(x0 + XT, g.kxn);
-  const int nl = x1 - x0;
   const int sv = GRAD ? (v == 0 ? 0 : 2) : (v < 3 ? v : (v == 3 ? 4 : 3));
   constexpr int TBL = Tiles<T>::TBL_I;
   const C* src = ub + (size_t)sv * ubi_var_elems<T>(g.nab_i, N);
-  // line l, entry z: column x0 + l holds kz = 0..kc then -kc..-1 (count
+  // line of column x, entry z: column x holds kz = 0..kc then -kc..-1 (count
   // 2 kc + 1, mpisetup.f:322-357), so its cylinder index follows from
-  // colstart alone; pass 0 of the transform reads the entries straight from
-  // ub (consecutive z of a warp are consecutive columns), the cut band is zero
+  // colstart alone; the cut band is zero
   struct Line { int ac, kc, x; };
   auto begin = [&](int l) {
-    const int ac = __ldg(g.colstart + x0 + l);
-    return Line{ac, (__ldg(g.colstart + x0 + l + 1) - ac - 1) / 2, x0 + l};
+    const int x = x0 + l;
+    if (x >= g.kxn) return Line{0, -1, x};   // a line of the last panel beyond kxn: zero
+    const int ac = __ldg(g.colstart + x);
+    return Line{ac, (__ldg(g.colstart + x + 1) - ac - 1) / 2, x};
   };
   auto fetch = [&](const Line& s, int z) {
     if (z > s.kc && z < N - s.kc) return cmk<C>(0, 0);
@@ -397,30 +419,51 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
     }
     return conj_if<TCM>(val);
   };
-  // the last pass stores its outputs straight to uz: line l, entry z at
-  // ((v n + y) nzt + z / TZ) kxn + x0 + l) TZ + z % TZ (consecutive z of a
-  // warp fill whole 32-byte sectors)
-  const size_t vbase = ((size_t)v * N + y) * g.nzt;
-  constexpr size_t zstride = (size_t)kxn_of(N) * TZ;   // g.kxn, as a constant
-  auto sbegin = [&](int l) { return uz + (vbase * g.kxn + x0 + l) * TZ; };
-  auto store = [&](C* d, int base, const C* vals, auto Rc, auto NSc) {
-    constexpr int R = decltype(Rc)::value, NS = decltype(NSc)::value;
-    static_assert(NS % TZ == 0, "last-pass stride must keep z % TZ");
-    C* p = d + ((unsigned)base / TZ) * zstride + (unsigned)base % TZ;
-#pragma unroll
-    for (int r = 0; r < R; r++) p[(size_t)(r * (NS / TZ)) * zstride] = vals[r];
-  };
+  C* const plane = uz + ((size_t)v * N + y) * uz_slab<T>(N);
   if constexpr (TCM) {
+    static_assert(kTcXT2 >= 4, "an operand tile overlays four lines");
+    constexpr int THREADS = Launch<T, N, XT>::THREADS, L = LS<T, N>::value;
+    C* buf = tw + PL::TWSIZE;
+    const int nl = min(x0 + XT, g.kxn) - x0;
     tc::Work w;
     constexpr int NCOL = tc_cols(XT);
     tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(buf + XT * L), tca);
     tc::fft1024<THREADS>(
         nl, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * L * sizeof(C)), begin,
-        [&](const Line& s, int z) { return fix(s, z, fetch(s, z)); }, sbegin,
-        [&](C* d, int z, C v) { d[((unsigned)z / TZ) * zstride + (unsigned)z % TZ] = cconj(v); });
+        [&](const Line& s, int z) { return fix(s, z, fetch(s, z)); }, [&](int l) { return x0 + l; },
+        [&](int x, int z, C val) { plane[uz_at<T, N>(x, z)] = cconj(val); });
     tc::teardown<NCOL>(w);
   } else {
-    fft_lines_load_store<T, N, THREADS, true>(buf, nl, L, tw, begin, fetch, fix, sbegin, store);
+    constexpr int R0 = PL::rad(0), E = PL::E, P = PL::P, RL = PL::rad(PL::NPASS - 1);
+    const int l = threadIdx.x / P, t = threadIdx.x % P;
+    const Line s = begin(l);
+    C val[E];
+#pragma unroll
+    for (int q = 0; q < E / R0; q++)
+#pragma unroll
+      for (int r = 0; r < R0; r++) val[q * R0 + r] = fetch(s, t + q * P + r * (N / R0));
+#pragma unroll
+    for (int q = 0; q < E / R0; q++)
+#pragma unroll
+      for (int r = 0; r < R0; r++) val[q * R0 + r] = fix(s, t + q * P + r * (N / R0), val[q * R0 + r]);
+    cp_async_wait_all();
+    __syncthreads();   // the twiddles
+    const unsigned o = (l / PA::PW) * PA::BYTES + (l % PA::PW) * 16;
+    panel_fft<T, N, true>(smem_raw, o, t, tw, val);
+    panel_store<T, N, RL>(smem_raw, o, t, val);
+    // every thread's writes before the copy engine's reads
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int npan = min(ZL::PPB, ZL::NPAN - (int)blockIdx.y * ZL::PPB);
+      C* dst = plane + (size_t)blockIdx.y * ZL::PPB * PA::ELEMS;
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst),
+                   "r"((unsigned)__cvta_generic_to_shared(smem_raw)), "r"(npan * PA::BYTES)
+                   : "memory");
+      asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+      // the block's shared memory must outlive the copy's reads
+      asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+    }
   }
 }
 
@@ -433,6 +476,30 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* addr, double 
   atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
+// The z-pencil slots of a K3 tile: pair p of tile zt is the real lines z =
+// zt TZ + 2 p and the next one; element x of the first sits at element
+// off(x) of its plane, the second's BS elements on.
+template <typename T, int N> struct XPair {
+  using PA = Panel<T, N>;
+  static constexpr int BS = PA::DBL ? PA::ROW : 1;
+  unsigned row, s;   // element of the pair's row in a panel, slot rotation
+  __device__ __forceinline__ XPair(int zt, int p) {
+    const unsigned rho = (unsigned)(zt * Tiles<T>::TZ + 2 * p) / PA::ZS;
+    row = rho * PA::ROW;
+    s = PA::sw(rho);
+  }
+  __device__ __forceinline__ size_t off(int x) const {
+    return (size_t)((unsigned)x / PA::PW) * PA::ELEMS + row + (((unsigned)x % PA::PW) ^ s) * PA::ZS;
+  }
+  // off(t + P m) for P a multiple of the panel width: off(t) + m STEP
+  static constexpr int P = FFTPlan<T, N>::P;
+  static constexpr bool STRIDE = P % PA::PW == 0;
+  static constexpr size_t STEP = STRIDE ? (size_t)(P / PA::PW) * PA::ELEMS : 0;
+  __device__ __forceinline__ size_t off(size_t o0, int t, int m) const {
+    return STRIDE ? o0 + m * STEP : off(t + P * m);
+  }
+};
+
 template <typename T, int N>
 __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int nbuf, int L,
                                              C2<T>* __restrict__ uz, int slot0, int y, int zt,
@@ -442,6 +509,7 @@ __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int
   const int kxn = g.kxn;
   // thread -> fixed pair p, x strided by blockDim/NPAIR (no runtime division)
   const int p = threadIdx.x % NPAIR, x0 = threadIdx.x / NPAIR, xs = blockDim.x / NPAIR;
+  const XPair<T, N> xp(zt, p);
   for (int b = 0; b < nbuf; b++)
   for (int x = x0; x < kxn; x += xs) {
     const C* line = buf + (b * NPAIR + p) * L;
@@ -449,9 +517,9 @@ __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int
     const C Yn = line[padl<C, N>(x == 0 ? 0 : N - x)];
     const C A = cmk<C>((Y.x + Yn.x) * half_factor, (Y.y - Yn.y) * half_factor);
     const C B = cmk<C>((Y.y + Yn.y) * half_factor, (Yn.x - Y.x) * half_factor);
-    C* dst = uz + ((((size_t)(slot0 + b) * N + y) * g.nzt + zt) * kxn + x) * TZ + 2 * p;
+    C* dst = uz + ((size_t)(slot0 + b) * N + y) * uz_slab<T>(N) + xp.off(x);
     dst[0] = A;
-    dst[1] = B;
+    dst[XPair<T, N>::BS] = B;
   }
 }
 
@@ -469,6 +537,7 @@ __device__ __forceinline__ void xchain_pack(const Geo& g, const C2<T>* __restric
   constexpr int XI = (N / 2 + XST - 1) / XST;
   const int kxn = g.kxn;
   const int p = threadIdx.x % NPAIR, xth = threadIdx.x / NPAIR;
+  const XPair<T, N> xp(zt, p);
   C A[NV][XI], B[NV][XI];
 #pragma unroll
   for (int v = 0; v < NV; v++)
@@ -476,14 +545,14 @@ __device__ __forceinline__ void xchain_pack(const Geo& g, const C2<T>* __restric
     for (int i = 0; i < XI; i++) {
       const int x = xth + i * XST;
       if (x < kxn) {
-        const C* src = uz + ((((size_t)(v0 + v) * N + y) * g.nzt + zt) * kxn + x) * TZ + 2 * p;
+        const C* src = uz + ((size_t)(v0 + v) * N + y) * uz_slab<T>(N) + xp.off(x);
         if constexpr (sizeof(C) == 8) {
           const float4 q = *reinterpret_cast<const float4*>(src);
           A[v][i] = cmk<C>(q.x, q.y);
           B[v][i] = cmk<C>(q.z, q.w);
         } else {
           A[v][i] = src[0];
-          B[v][i] = src[1];
+          B[v][i] = src[XPair<T, N>::BS];
         }
       }
     }
@@ -543,7 +612,9 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
     const int l = l0 + lr;
     const bool act = l < NV * NPAIR;
     const int v = act ? l / NPAIR : 0, p = l % NPAIR;
-    const C* col = uz + (((size_t)(v0 + v) * N + y) * g.nzt + zt) * (size_t)kxn * TZ + 2 * p;
+    const XPair<T, N> xp(zt, p);
+    const C* col = uz + ((size_t)(v0 + v) * N + y) * uz_slab<T>(N);
+    const size_t o0 = xp.off(t);
     C a[H], b[H];
 #pragma unroll
     for (int m = 0; m < H; m++) {
@@ -552,12 +623,12 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
       b[m] = cmk<C>(0, 0);
       if (act && x < kxn) {
         if constexpr (sizeof(C) == 8) {
-          const float4 q = *reinterpret_cast<const float4*>(col + (size_t)x * TZ);
+          const float4 q = *reinterpret_cast<const float4*>(col + xp.off(o0, t, m));
           a[m] = cmk<C>(q.x, q.y);
           b[m] = cmk<C>(q.z, q.w);
         } else {
-          a[m] = col[(size_t)x * TZ];
-          b[m] = col[(size_t)x * TZ + 1];
+          a[m] = col[xp.off(o0, t, m)];
+          b[m] = col[xp.off(o0, t, m) + XPair<T, N>::BS];
         }
       }
     }
@@ -624,7 +695,9 @@ __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf
       for (int m = 0; m < E; m++) v[m] = cmk<C>(0, 0);
     }
     const int b = act ? l / NPAIR : 0, p = l % NPAIR;
-    C* col = uz + (((size_t)b * N + y) * g.nzt + zt) * (size_t)kxn * TZ + 2 * p;
+    const XPair<T, N> xp(zt, p);
+    C* col = uz + ((size_t)b * N + y) * uz_slab<T>(N);
+    const size_t o0 = xp.off(t);
 #pragma unroll
     for (int m = 0; m < H; m++) {
       const int x = t + P * m;
@@ -636,10 +709,10 @@ __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf
         const T ax = (Y.x + Yn.x) * half_factor, ay = (Y.y - Yn.y) * half_factor;
         const T bx = (Y.y + Yn.y) * half_factor, by = (Yn.x - Y.x) * half_factor;
         if constexpr (sizeof(C) == 8) {
-          *reinterpret_cast<float4*>(col + (size_t)x * TZ) = make_float4(ax, ay, bx, by);
+          *reinterpret_cast<float4*>(col + xp.off(o0, t, m)) = make_float4(ax, ay, bx, by);
         } else {
-          col[(size_t)x * TZ] = cmk<C>(ax, ay);
-          col[(size_t)x * TZ + 1] = cmk<C>(bx, by);
+          col[xp.off(o0, t, m)] = cmk<C>(ax, ay);
+          col[xp.off(o0, t, m) + XPair<T, N>::BS] = cmk<C>(bx, by);
         }
       }
     }
@@ -790,47 +863,29 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
 
 // ---------------------------------------------------------------------------
 // K4: z forward FFT + derivative combination + cylinder pack into ub (TB_F)
-// grid (n, ceil(kxn/k4_xt)).  Output slots: 0 = d/dx(u^2-v^2)+d/dz(uw) partial,
+// Output slots: 0 = d/dx(u^2-v^2)+d/dz(uw) partial,
 // 1 = uv, 2 = d/dx(uw)+d/dz(w^2-v^2), 3 = vw (y derivatives added in K5).
 // ---------------------------------------------------------------------------
-template <typename T, int N, int XT>
-__device__ __forceinline__ void zfwd_load(const Geo& g, const C2<T>* __restrict__ uz, int slot, int y0, int ny,
-                                          int x0, int nl, C2<T>* buf, int L) {
-  // lines l = yy*nl + xl, rows y0+yy, columns x0+xl; full tiles (nl = XT)
-  // take the loop with compile-time divisors
-  constexpr int TZ = Tiles<T>::TZ;
-  auto copy = [&](auto nlc, const C2<T>* src, C2<T>* b) {
-    constexpr int NLC = decltype(nlc)::value;
-    const unsigned w = (NLC > 0 ? NLC : nl) * TZ;
-    const unsigned cnt = (NLC > 0 ? NLC : nl) * N;
-    for (unsigned e = threadIdx.x; e < cnt; e += blockDim.x) {
-      const unsigned zt = e / w, rem = e % w, l = rem / TZ, zz = rem % TZ;
-      cp_async_elem(b + l * L + padl<C2<T>, N>(zt * TZ + zz), src + ((size_t)zt * g.kxn + l) * TZ + zz);
-    }
-  };
-  for (int yy = 0; yy < ny; yy++) {
-    const size_t vbase = ((size_t)slot * N + y0 + yy) * g.nzt;
-    const C2<T>* src = uz + (vbase * g.kxn + x0) * TZ;
-    C2<T>* b = buf + yy * nl * L;
-    if (nl == XT)
-      copy(std::integral_constant<int, XT>(), src, b);
-    else
-      copy(std::integral_constant<int, 0>(), src, b);
+// tensor-core form: the nl lines from x0 of one field at row y to buf
+template <typename T, int N>
+__device__ __forceinline__ void zfwd_load(const C2<T>* __restrict__ uz, int slot, int y, int x0, int nl, C2<T>* buf,
+                                          int L) {
+  const C2<T>* plane = uz + ((size_t)slot * N + y) * uz_slab<T>(N);
+  for (unsigned e = threadIdx.x; e < (unsigned)nl * N; e += blockDim.x) {
+    const unsigned z = e % N, l = e / N;
+    cp_async_elem(buf + l * L + padl<C2<T>, N>(z), plane + uz_at<T, N>(x0 + l, z));
   }
 }
 
 template <typename T, int N, int MODE, int XT>
 __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const C2<T>* s1, int L,
-                                           C2<T>* __restrict__ ub, int slot, int y0, int /*ny*/, int x0, int x1,
+                                           C2<T>* __restrict__ ub, int slot, int y0, int x0, int x1,
                                            T b11, T b33) {
-  constexpr int ny = Tiles<T>::YT4;
-  // the ny rows of one block column are adjacent in ub: write them together
   using C = C2<T>;
   constexpr int TB = Tiles<T>::TBL_F;   // runs of the forward ub layout
-  const int nl = x1 - x0;
   const int abeg = __ldg(g.colstart + x0), aend = __ldg(g.colstart + x1);
   const int as = abeg - (abeg % TB);                      // first block boundary
-  const int cnt = ((aend - as + TB - 1) / TB) * TB * ny;  // whole blocks x rows
+  const int cnt = ((aend - as + TB - 1) / TB) * TB;  // whole blocks
   C* dst = ub + (size_t)slot * ubf_var_elems<T>(g.nab_f, N);
   // column starts of the XT lines: x and z of a cylinder index follow from
   // them (column x0 + j holds kz = 0..kc then -kc..-1)
@@ -838,17 +893,14 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
 #pragma unroll
   for (int j = 0; j <= XT; j++) csr[j] = __ldg(g.colstart + min(x0 + j, g.kxn));
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-    // e -> (block q, row yy, column a): the ny rows of a block are adjacent
-    // in memory, so consecutive threads write consecutive addresses
-    const int q = e / (TB * ny), r = e % (TB * ny);
-    const int yy = r / TB, a = as + q * TB + r % TB;
+    const int a = as + e;
     if (a < abeg || a >= aend) continue;
     int lx = 0, c0 = csr[0], c1 = csr[1];
 #pragma unroll
     for (int j = 1; j < XT; j++)
       if (a >= csr[j]) { lx = j; c0 = csr[j]; c1 = csr[j + 1]; }
     const int kc = (c1 - c0 - 1) / 2, ia = a - c0;
-    const int x = x0 + lx, z = ia <= kc ? ia : ia + N - (2 * kc + 1), l = yy * nl + lx;
+    const int x = x0 + lx, z = ia <= kc ? ia : ia + N - (2 * kc + 1), l = lx;
     const int i = l * L + padl<C, N>(z);
     C out;
     if constexpr (MODE == 0) {          // i kx P1 + i b33 kz P5   (s1 = P1, s0 = P5)
@@ -865,164 +917,217 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
       out = s1[i];
     } else {                            // MODE 4: s0 to this slot and s1 to slot + 2
       out = s0[i];
-      dst[2 * ubf_var_elems<T>(g.nab_f, N) + ((size_t)((unsigned)a / TB) * N + y0 + yy) * TB + ((unsigned)a % TB)] =
+      dst[2 * ubf_var_elems<T>(g.nab_f, N) + ((size_t)((unsigned)a / TB) * N + y0) * TB + ((unsigned)a % TB)] =
           s1[i];
     }
-    dst[((size_t)((unsigned)a / TB) * N + y0 + yy) * TB + ((unsigned)a % TB)] = out;
+    dst[((size_t)((unsigned)a / TB) * N + y0) * TB + ((unsigned)a % TB)] = out;
   }
 }
 
-// K4 with register-fed transforms (the FP32 and FP64 stage kernels): pass 0
-// of every z transform takes its operands straight from uz, and the last pass
-// of P1, P3, P2, P4 (and of the scalar term) writes the cylinder entries of ub
-// from registers (consecutive z of a warp are consecutive cylinder indices),
-// so shared memory carries only the exchanges between passes and the P5
-// lines that the derivative combinations of P1 and P3 read.
-// Phase 1: P5, P1, P3 (P5's last pass in shared memory; then P1 -> ub slot 0,
-// P3 -> slot 2); phase 2: P2 -> slot 1, P4 -> slot 3 (uz slot 5 -> ub slot 4
-// with a scalar).  Field f of x line xl is line f nl + xl of its phase.
-template <typename T, int N, int NC, int THREADS>
-__device__ __forceinline__ void zfwd_fused(const Geo& g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub,
-                                           C2<T>* buf, const C2<T>* tw, int y, int x0, int nl, T b11, T b33) {
+// K4 of the FP32 and FP64 stage kernels.  A tile is PPB panels of x lines at one
+// y; its five fields (six with a scalar) come one after the other, as whole
+// contiguous panels, through three shared-memory buffers (16-byte cp.async,
+// the copies of the next one or two fields in flight while one is transformed,
+// across tiles), and each line is transformed in place by its own group of P
+// threads.  P5 comes first and stays in buffer 0 for the derivative
+// combinations of P1 and P3 (each thread reads back the elements it wrote);
+// then P1 -> ub slot 0, P3 -> slot 2, P2 -> slot 1, P4 -> slot 3 (uz slot 5 ->
+// ub slot 4 with a scalar).  The last pass writes the cylinder entries from
+// registers: consecutive z of a warp are consecutive cylinder indices.
+// One block barrier per field: it makes the field's copy visible, and frees
+// the buffer of the field before.
+template <typename T, int N, int NC, int PPBO>
+__device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub,
+                                            unsigned char* smem, const C2<T>* __restrict__ tw_g, int ntiles, T b11,
+                                            T b33) {
   using C = C2<T>;
   using PL = FFTPlan<T, N>;
-  static_assert(Tiles<T>::YT4 == 1, "one y row per block");
-  static_assert(PL::NPASS >= 2, "load and store passes must differ");
-  constexpr int TZ = Tiles<T>::TZ, TB = Tiles<T>::TBL_F, L = LS<T, N>::value;
-  constexpr size_t zstride = (size_t)kxn_of(N) * TZ;   // g.kxn, as a constant
+  using PA = Panel<T, N>;
+  using ZL = ZLaunch<T, N, PPBO>;
+  constexpr int TB = Tiles<T>::TBL_F, E = PL::E, P = PL::P, R0 = PL::rad(0);
+  constexpr int RL = PL::rad(PL::NPASS - 1), NSL = PL::ns(PL::NPASS - 1), H = RL / 2;
+  static_assert(H * NSL == N / 2, "the halves of the last pass are the signs of kz");
+  constexpr int LT = ilog2c(TB), ITEMS = 5 + NC;
+  C* tw = reinterpret_cast<C*>(smem + 3 * ZL::BUF);
   const size_t var = ubf_var_elems<T>(g.nab_f, N);
-  // uz field `slot` of x line x0 + xl at row y: entry z at (z / TZ) zstride + z % TZ
-  struct In { const C* src; };
-  auto in_line = [&](int slot, int xl) {
-    return In{uz + ((((size_t)slot * N + y) * g.nzt) * g.kxn + x0 + xl) * TZ};
-  };
-  auto fetch = [&](const In& s, int z) { return __ldg(s.src + ((unsigned)z / TZ) * zstride + (unsigned)z % TZ); };
-  auto nofix = [](const In&, int, C v) { return v; };
-  // ub slot of x line x0 + xl: column x holds kz = 0..kc then -kc..-1 from
-  // cylinder index c0 (mpisetup.f:322-357); mode 0: i kx P1 + i b33 kz P5,
-  // mode 1: i b11 kx P5 + i kz P3, mode 2: the value itself
-  struct Out { C* dst; const C* p5; int x, c0, kc, mode; };
-  auto out_line = [&](int slot, int xl, int mode) {
-    const int c0 = __ldg(g.colstart + x0 + xl);
-    return Out{ub + (size_t)slot * var, buf + (size_t)xl * L, x0 + xl, c0,
-               (__ldg(g.colstart + x0 + xl + 1) - c0 - 1) / 2, mode};
-  };
-  auto store = [&](const Out& s, int base, const C* v, auto Rc, auto NSc) {
-    constexpr int R = decltype(Rc)::value, NS = decltype(NSc)::value;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int z = base + r * NS;
-      if (z > s.kc && z < N - s.kc) continue;
-      C out = v[r];
-      if (s.mode == 0) {
-        const T kx = T(s.x), bk3 = b33 * T(kwave<N>(z));
-        const C p5 = s.p5[padl<C, N>(z)];
-        out = cmk<C>(-kx * v[r].y - bk3 * p5.y, kx * v[r].x + bk3 * p5.x);
-      } else if (s.mode == 1) {
-        const T bk1 = b11 * T(s.x), kz = T(kwave<N>(z));
-        const C p5 = s.p5[padl<C, N>(z)];
-        out = cmk<C>(-bk1 * p5.y - kz * v[r].y, bk1 * p5.x + kz * v[r].x);
-      }
-      const int a = s.c0 + (z <= s.kc ? z : z - N + 2 * s.kc + 1);
-      s.dst[((size_t)((unsigned)a / TB) * N + y) * TB + ((unsigned)a % TB)] = out;
+  const int l = threadIdx.x / P, t = threadIdx.x % P;
+  // field of the it-th item: uz slot, ub slot
+  auto in_slot = [](int it) { return it == 0 ? 4 : it == 1 ? 0 : it == 2 ? 2 : it == 3 ? 1 : it == 4 ? 3 : 5; };
+  auto out_slot = [](int it) { return it == 1 ? 0 : it == 2 ? 2 : it == 3 ? 1 : it == 4 ? 3 : 4; };
+  // tiles of one panel column follow one another in y: the 64-byte runs that
+  // neighbouring y write to ub meet in L2
+  auto copy = [&](int buf, int it, int tile) {
+    if (tile < ntiles) {
+      const int box = tile / (ZL::TILES * N), rem = tile % (ZL::TILES * N), sp = rem / N, y = rem % N;
+      const unsigned bytes = min(ZL::PPB, ZL::NPAN - sp * ZL::PPB) * PA::BYTES;
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(
+          uz + box * g.zbox + ((size_t)in_slot(it) * N + y) * uz_slab<T>(N) + (size_t)sp * ZL::PPB * PA::ELEMS);
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(smem + buf * ZL::BUF);
+      for (unsigned o = threadIdx.x * 16; o < bytes; o += ZL::THREADS * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + o), "l"(src + o) : "memory");
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  // phase 1
-  fft_pass0_load<T, N, THREADS>(
-      buf, 3 * nl, L, [&](int l) { return in_line(l < nl ? 4 : (l < 2 * nl ? 0 : 2), l % nl); }, fetch, nofix);
-  cp_async_wait_all();
-  __syncthreads();
-  fft_passes_until<T, N, THREADS, 1, PL::NPASS - 1>(buf, 3 * nl, L, tw);
-  fft_passes_until<T, N, THREADS, PL::NPASS - 1, PL::NPASS>(buf, nl, L, tw);
-  __syncthreads();   // P5 lines complete
-  fft_pass_last_store<T, N, THREADS>(buf + (size_t)nl * L, 2 * nl, L, tw,
-                                     [&](int l) { return l < nl ? out_line(0, l, 0) : out_line(2, l - nl, 1); },
-                                     store);
-  __syncthreads();   // every line of phase 1 read
-  // phase 2
-  constexpr int NV2 = 2 + NC;
-  fft_pass0_load<T, N, THREADS>(
-      buf, NV2 * nl, L, [&](int l) { return in_line(l < nl ? 1 : (l < 2 * nl ? 3 : 5), l % nl); }, fetch, nofix);
-  __syncthreads();
-  fft_passes_until<T, N, THREADS, 1, PL::NPASS - 1>(buf, NV2 * nl, L, tw);
-  fft_pass_last_store<T, N, THREADS>(
-      buf, NV2 * nl, L, tw,
-      [&](int l) { return out_line(l < nl ? 1 : (l < 2 * nl ? 3 : 4), l % nl, 2); }, store);
+  const int step = gridDim.x;
+  int w = 1;   // buffer of P1 and P2; 3 - w: of P3 and P4
+  load_twiddles<T, N>(tw, tw_g);
+  copy(0, 0, blockIdx.x);
+  copy(w, 1, blockIdx.x);
+  for (int tile = blockIdx.x; tile < ntiles; tile += step) {
+    const int box = tile / (ZL::TILES * N), rem = tile % (ZL::TILES * N), sp = rem / N, y = rem % N;
+    const int x = sp * ZL::LINES + l;
+    const bool act = x < g.kxn;
+    // column x holds kz = 0..kc then -kc..-1 from cylinder index c0
+    // (mpisetup.f:322-357)
+    const int c0 = act ? __ldg(g.colstart + x) : 0;
+    const int kc = act ? (__ldg(g.colstart + x + 1) - c0 - 1) / 2 : -1;
+    C* const dst0 = ub + box * g.bbox + (size_t)y * TB;
+    const unsigned line = (l / PA::PW) * PA::BYTES + (l % PA::PW) * 16;   // the line's place in a buffer
+#pragma unroll 1
+    for (int it = 0; it < ITEMS; it++) {
+      // copies in flight behind this item's: one, or none (items 2, 3 and the
+      // scalar's)
+      if (it == 2 || it == 3 || it == 5)
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      else
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      __syncthreads();
+      // refill what the item before has left
+      if (it == 0) {
+        copy(3 - w, 2, tile);
+      } else if (it == 2) {
+        copy(w, 3, tile);
+      } else if (it == 3) {
+        copy(3 - w, 4, tile);
+        copy(0, 0, tile + step);
+      } else if (it == 4) {
+        if constexpr (NC > 0) copy(w, 5, tile);
+        else copy(w, 1, tile + step);
+      } else if (it == 5) {
+        copy(3 - w, 1, tile + step);
+      }
+      const int buf = it == 0 ? 0 : (it == 2 || it == 4) ? 3 - w : w;
+      const unsigned o = buf * ZL::BUF + line;
+      C v[E];
+      panel_load<T, N, R0>(smem, o, t, v);
+      line_sync<P>();
+      panel_fft<T, N, false>(smem, o, t, tw, v);
+      if (it == 0) {
+        panel_store<T, N, RL>(smem, o, t, v);
+        continue;
+      }
+      if (it < 3) {
+        // i (a v + b P5): slot 0 a = kx, b = b33 kz; slot 2 a = kz, b = b11 kx
+        const T a0 = it == 1 ? T(x) : T(0), a1 = it == 1 ? T(0) : T(1);
+        const T d0 = it == 1 ? T(0) : b11 * T(x), d1 = it == 1 ? b33 : T(0);
+#pragma unroll
+        for (int q = 0; q < E / RL; q++) {
+          const int j = t + q * P;
+          C p5[RL];
+          panel_read<T, N, false, RL, NSL>(smem, line ^ PA::template off<false>(j), line, j, p5);
+#pragma unroll
+          for (int r = 0; r < RL; r++) {
+            const T kz = T(j + r * NSL - (r < H ? 0 : N));
+            const T ka = a0 + a1 * kz, kd = d0 + d1 * kz;
+            const C u = v[q * RL + r];
+            v[q * RL + r] = cmk<C>(-ka * u.y - kd * p5[r].y, ka * u.x + kd * p5[r].x);
+          }
+        }
+      }
+      C* const d = dst0 + out_slot(it) * var;
+#pragma unroll
+      for (int q = 0; q < E / RL; q++) {
+        const int j = t + q * P;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          // first half: z = j + r NS <= kc at cylinder index c0 + z; second half:
+          // z - N >= -kc at c0 + 2 kc + 1 + (z - N)
+          const int z0 = h == 0 ? j : j - N / 2;
+          const int a0 = h == 0 ? c0 + z0 : c0 + 2 * kc + 1 + z0;
+#pragma unroll
+          for (int r = 0; r < H; r++) {
+            const bool in = h == 0 ? z0 + r * NSL <= kc : z0 + r * NSL >= -kc;
+            long e;
+            if constexpr (NSL % TB == 0) {   // NS steps over whole runs of TB columns
+              e = (long)(a0 >> LT) * (N * TB) + (a0 & (TB - 1)) + (long)r * ((long)(NSL / TB) * N * TB);
+            } else {
+              const int a = a0 + r * NSL;
+              e = (long)(a >> LT) * (N * TB) + (a & (TB - 1));
+            }
+            if (in) d[e] = v[q * RL + h * H + r];
+          }
+        }
+      }
+    }
+    if constexpr (NC > 0) w = 3 - w;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// XTO > 0: XTO x lines per block instead of k4_xt (ensemble tuner)
-template <typename T, int N, int NC = 0, bool TCM = false, int XTO = 0>
-__global__ void __launch_bounds__(K4LaunchX<T, N, (XTO > 0 ? XTO : k4_xt(sizeof(T) == 8, N)), TCM>::THREADS,
-                                  K4LaunchX<T, N, (XTO > 0 ? XTO : k4_xt(sizeof(T) == 8, N)), TCM>::MINB)
-k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__ tw_g,
+// PPBO > 0: panels per block (ensemble tuner).  grid: the tiles (n y rows x
+// TILES x boxes), or as many blocks as stay resident; tensor-core form:
+// (n, lines / kTcXT4)
+template <typename T, int N, int NC = 0, bool TCM = false, int PPBO = 0>
+__global__ void __launch_bounds__(TCM ? Launch<T, N, 2 * kTcXT4, 1024>::THREADS : ZLaunch<T, N, PPBO>::THREADS,
+                                  TCM ? 2 : ZLaunch<T, N, PPBO>::MINB4)
+k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__ tw_g, int ntiles,
        T b11, T b33, TcArgs tca = TcArgs()) {
   // NC = 1: the scalar advection term (uz slot 5) goes to ub slot 4 without
   // derivatives (transform.f: i2f = 4+nc)
-  // grid (n / YT4, ceil(kxn / XT)): YT4 adjacent y rows x XT x lines
   using C = C2<T>;
-  constexpr int XT = XTO > 0 ? XTO : k4_xt(sizeof(T) == 8, N), YT = Tiles<T>::YT4, NLT = XT * YT;
-  static_assert(!TCM || NLT >= 4, "an operand tile overlays four lines of s0 or s1");
-  constexpr int THREADS = K4LaunchX<T, N, XT, TCM>::THREADS;
-  constexpr int L = LS<T, N>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* s0 = tw + FFTPlan<T, N>::TWSIZE;
-  C* s1 = s0 + NLT * L;
-  load_twiddles<T, N>(tw, tw_g);
-  // grid (n / YT4, ceil(kxn / XT), boxes)
-  const int y0 = blockIdx.x * YT, x0 = blockIdx.y * XT, box = blockIdx.z;
-  uz += box * g.zbox;
-  ub += box * g.bbox;
-  const int x1 = min(x0 + XT, g.kxn);
-  const int nl = x1 - x0;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
   if constexpr (!TCM) {
-    zfwd_fused<T, N, NC, THREADS>(g, uz, ub, s0, tw, y0, x0, nl, b11, b33);
+    zfwd_panels<T, N, NC, PPBO>(g, uz, ub, smem_raw, tw_g, ntiles, b11, b33);
   } else {
     // tensor-core form: rounds of two fields through shared memory
-    constexpr int NCOL = tc_cols(2 * NLT);
+    constexpr int XT = kTcXT4, THREADS = Launch<T, N, 2 * XT, 1024>::THREADS, L = LS<T, N>::value;
+    static_assert(XT >= 4, "an operand tile overlays four lines of s0 or s1");
+    C* tw = reinterpret_cast<C*>(smem_raw);
+    C* s0 = tw + FFTPlan<T, N>::TWSIZE;
+    C* s1 = s0 + XT * L;
+    load_twiddles<T, N>(tw, tw_g);
+    const int y = blockIdx.x, x0 = blockIdx.y * XT, x1 = min(x0 + XT, g.kxn), nl = x1 - x0;
+    constexpr int NCOL = tc_cols(2 * XT);
     tc::Work w;
-    tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(s1 + NLT * L), tca);
-    const int nt = nl * YT;
+    tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(s1 + XT * L), tca);
+    auto both = [&]() {
+      if (nl == XT) {
+        lines_fft<T, N, THREADS, TCM>(s0, 2 * XT, L, tw, w);
+      } else {
+        lines_fft<T, N, THREADS, TCM>(s0, nl, L, tw, w);
+        lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
+      }
+    };
     // round 1: P5 -> s0, P1 -> s1
-    zfwd_load<T, N, XT>(g, uz, 4, y0, YT, x0, nl, s0, L);
-    zfwd_load<T, N, XT>(g, uz, 0, y0, YT, x0, nl, s1, L);
+    zfwd_load<T, N>(uz, 4, y, x0, nl, s0, L);
+    zfwd_load<T, N>(uz, 0, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
-    if (nl == XT) {
-      lines_fft<T, N, THREADS, TCM>(s0, 2 * NLT, L, tw, w);
-    } else {
-      lines_fft<T, N, THREADS, TCM>(s0, nt, L, tw, w);
-      lines_fft<T, N, THREADS, TCM>(s1, nt, L, tw, w);
-    }
-    zfwd_store<T, N, 0, XT>(g, s0, s1, L, ub, 0, y0, YT, x0, x1, b11, b33);
+    both();
+    zfwd_store<T, N, 0, XT>(g, s0, s1, L, ub, 0, y, x0, x1, b11, b33);
     __syncthreads();
     // round 2: P3 -> s1
-    zfwd_load<T, N, XT>(g, uz, 2, y0, YT, x0, nl, s1, L);
+    zfwd_load<T, N>(uz, 2, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
-    lines_fft<T, N, THREADS, TCM>(s1, nt, L, tw, w);
-    zfwd_store<T, N, 1, XT>(g, s0, s1, L, ub, 2, y0, YT, x0, x1, b11, b33);
+    lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
+    zfwd_store<T, N, 1, XT>(g, s0, s1, L, ub, 2, y, x0, x1, b11, b33);
     __syncthreads();
     // round 3: P2 -> s0, P4 -> s1
-    zfwd_load<T, N, XT>(g, uz, 1, y0, YT, x0, nl, s0, L);
-    zfwd_load<T, N, XT>(g, uz, 3, y0, YT, x0, nl, s1, L);
+    zfwd_load<T, N>(uz, 1, y, x0, nl, s0, L);
+    zfwd_load<T, N>(uz, 3, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
-    if (nl == XT) {
-      lines_fft<T, N, THREADS, TCM>(s0, 2 * NLT, L, tw, w);
-    } else {
-      lines_fft<T, N, THREADS, TCM>(s0, nt, L, tw, w);
-      lines_fft<T, N, THREADS, TCM>(s1, nt, L, tw, w);
-    }
+    both();
     // P2 -> ub slot 1 and P4 -> ub slot 3 in one pass over the cylinder indices
-    zfwd_store<T, N, 4, XT>(g, s0, s1, L, ub, 1, y0, YT, x0, x1, b11, b33);
+    zfwd_store<T, N, 4, XT>(g, s0, s1, L, ub, 1, y, x0, x1, b11, b33);
     if constexpr (NC > 0) {
       __syncthreads();
-      zfwd_load<T, N, XT>(g, uz, 5, y0, YT, x0, nl, s1, L);
+      zfwd_load<T, N>(uz, 5, y, x0, nl, s1, L);
       cp_async_wait_all();
       __syncthreads();
-      lines_fft<T, N, THREADS, TCM>(s1, nt, L, tw, w);
-      zfwd_store<T, N, 3, XT>(g, s0, s1, L, ub, 4, y0, YT, x0, x1, b11, b33);
+      lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
+      zfwd_store<T, N, 3, XT>(g, s0, s1, L, ub, 4, y, x0, x1, b11, b33);
     }
     tc::teardown<NCOL>(w);
   }

@@ -81,7 +81,7 @@ static Plan plan_for(const Geometry& g) {
   const size_t cs = sizeof(C2<T>);
   const size_t nab_i = (g.xz_tot + TL::TB_I - 1) / TL::TB_I, nab_f = (g.xz_tot + TL::TB_F - 1) / TL::TB_F;
   const size_t ub_el = std::max(3 * ubi_var_elems<T>((int)nab_i, N), 4 * ubf_var_elems<T>((int)nab_f, N));
-  const size_t uz_el = (size_t)5 * N * N * g.kxn;
+  const size_t uz_el = (size_t)5 * N * uz_slab<T>(N);
   const size_t tab = 2 * (N / 2 + 1 + 2 * N) * cs + (N / 2 + 1 + 2 * N) * sizeof(T);
   Plan p;
   size_t o = 0;
@@ -187,27 +187,20 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   unsigned long long* vmx = (unsigned long long*)(base + pl.velmax);
   constexpr int L = LS<T, N>::value;
   constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
-  const int kxn = g.kxn;
   {
     constexpr int TH = K1Launch<T, N>::THREADS;
     k_yinv<T, N><<<dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st>>>(geo, stb, u, ub, twd);
   }
-  {
-    constexpr int TH = Launch<T, N, TL::XT2>::THREADS;
-    k_zinv<T, N><<<dim3(N, (kxn + TL::XT2 - 1) / TL::XT2, 3), TH, TWB + sizeof(C) * TL::XT2 * L, st>>>(geo, ub, uz,
-                                                                                                       twd);
-  }
+  using ZL = ZLaunch<T, N, 0>;
+  k_zinv<T, N><<<dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st>>>(geo, ub, uz, twd);
   {
     constexpr int TH = K3Launch<T, N, 0>::THREADS;
     k_xchain<T, N><<<dim3(geo.nzt, N), TH, K3Launch<T, N, 0>::SMEM, st>>>(
         geo, uz, twd, stb.b11, stb.b22, stb.b33, vmx, kstep == 1 ? 1 : 0);
   }
-  {
-    constexpr int TH = K4Launch<T, N>::THREADS;
-    constexpr int XT4 = k4_xt(sizeof(T) == 8, N);
-    k_zfwd<T, N><<<dim3(N / TL::YT4, (kxn + XT4 - 1) / XT4), TH, K4Launch<T, N>::SMEM, st>>>(
-        geo, uz, ub, twd, stb.b11, stb.b33);
-  }
+  const int tiles = N * ZL::TILES;
+  k_zfwd<T, N><<<std::min(tiles, 148 * ZL::MINB4), ZL::THREADS, ZL::SMEM4, st>>>(geo, uz, ub, twd, tiles, stb.b11,
+                                                                                stb.b33);
   {
     constexpr int TH = K5Launch<T, N, 0>::THREADS;
     if (kstep == 1)
