@@ -139,7 +139,7 @@ template <typename T, int N> struct EnsImpl {
       case 2: k2<4>(e, g, ub, uz, tw, st, nb); break;
       default: k2<1>(e, g, ub, uz, tw, st, nb);
     }
-    k_xchain<T, N><<<dim3(e.nzt, N, nb), K3Launch<T, N, 0>::THREADS, I::sm3(), e.stream>>>(
+    k_xchain<T, N><<<dim3(N / K3Launch<T, N, 0>::TZ, N, nb), K3Launch<T, N, 0>::THREADS, I::sm3(), e.stream>>>(
         g, uz, tw, st.b11, st.b22, st.b33, e.d_velmax + b0, kstep == 1 ? 1 : 0);
     switch (kTiles ? e.k4v : 0) {
       case 1: k4<2>(e, g, uz, ub, tw, st, nb); break;

@@ -358,7 +358,7 @@ template <typename T, int N, int NC> struct Impl {
       CK(cudaFuncSetAttribute(k_zinv<T, N, NC, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm2tc()));
       CK(cudaFuncSetAttribute(k_xchain<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)K3Launch<T, N, NC>::SMEM_TC));
+                              (int)K3Launch<T, N, NC, true>::SMEM_TC));
       CK(cudaFuncSetAttribute(k_zfwd<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm4tc()));
       CK(cudaFuncSetAttribute(k_yfwd<T, N, 1, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -534,7 +534,7 @@ template <typename T, int N, int NC> struct Impl {
       // mean-gradient coefficients cb = beta * grad (init.f:42-45)
       const T cb1 = (T)(c.p.beta1 * c.p.grad[0]), cb2 = (T)(c.p.beta2 * c.p.grad[1]),
               cb3 = (T)(c.p.beta3 * c.p.grad[2]);
-      k_xchain<T, N, NC><<<dim3(c.nzt, N), TH, sm3(), c.stream>>>(g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax,
+      k_xchain<T, N, NC><<<dim3(N / K3Launch<T, N, NC>::TZ, N), TH, sm3(), c.stream>>>(g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax,
                                                                     kstep == 1 ? 1 : 0, cb1, cb2, cb3);
       prof_mark(c, s, 2, 1);
     }
@@ -572,7 +572,7 @@ template <typename T, int N, int NC> struct Impl {
     prof_mark(c, s, 2, 0);
     const T cb1 = (T)(c.p.beta1 * c.p.grad[0]), cb2 = (T)(c.p.beta2 * c.p.grad[1]),
             cb3 = (T)(c.p.beta3 * c.p.grad[2]);
-    k_xchain<T, N, NC, true><<<dim3(c.nzt, N), K3Launch<T, N, NC>::THREADS, K3Launch<T, N, NC>::SMEM_TC,
+    k_xchain<T, N, NC, true><<<dim3(N / K3Launch<T, N, NC, true>::TZ, N), K3Launch<T, N, NC, true>::THREADS, K3Launch<T, N, NC, true>::SMEM_TC,
                                c.stream>>>(g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1,
                                            cb2, cb3, ta);
     prof_mark(c, s, 2, 1);

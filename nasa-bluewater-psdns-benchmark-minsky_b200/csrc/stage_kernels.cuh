@@ -101,8 +101,8 @@ template <typename T> struct StageTables {
 };
 
 // per-precision tile sizes: TB_I = columns per K1 block (64 B runs in ub
-// for K2), TB_F = columns per K5 block, TZ = z lines per K3 tile
-// (whole rows of the z-pencil panels).
+// for K2), TB_F = columns per K5 block, TZ = z lines per tile of the spline and
+// moment kernels.
 // Eight lines per K1 block keep two to three blocks resident per SM, so that
 // one block's copies overlap another's transforms; sixteen-line blocks (one
 // per SM) measured slower.
@@ -381,7 +381,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
   using ZL = ZLaunch<T, N, PPBO>;
   using PA = Panel<T, N>;
   constexpr int XT = TCM ? kTcXT2 : ZL::LINES;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw + (TCM ? 0 : ZL::BUF));
   load_twiddles<T, N>(tw, tw_g);
   // grid (n, lines / XT, fields * boxes)
@@ -438,10 +438,29 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
     const int l = threadIdx.x / P, t = threadIdx.x % P;
     const Line s = begin(l);
     C val[E];
+    constexpr int S0 = N / R0, H = R0 / 2, LT = ilog2c(TBL);
+    if constexpr (S0 % TBL == 0 && H * S0 == N / 2) {
+      // steps of S0 cover whole runs of TBL columns, and the first H operands
+      // are the entries z < n/2: two addresses a thread, the rest constants
 #pragma unroll
-    for (int q = 0; q < E / R0; q++)
+      for (int q = 0; q < E / R0; q++)
 #pragma unroll
-      for (int r = 0; r < R0; r++) val[q * R0 + r] = fetch(s, t + q * P + r * (N / R0));
+        for (int h = 0; h < 2; h++) {
+          const int z0 = h == 0 ? t + q * P : t + q * P - N / 2;   // kz of the half's first operand
+          const int a0 = h == 0 ? s.ac + z0 : s.ac + 2 * s.kc + 1 + z0;
+          const C* p0 = src + (long)(a0 >> LT) * (N * TBL) + (a0 & (TBL - 1)) + y * TBL;
+#pragma unroll
+          for (int r = 0; r < H; r++) {
+            const bool in = h == 0 ? z0 + r * S0 <= s.kc : z0 + r * S0 >= -s.kc;
+            val[q * R0 + h * H + r] = in ? __ldg(p0 + (long)r * ((long)(S0 / TBL) * N * TBL)) : cmk<C>(0, 0);
+          }
+        }
+    } else {
+#pragma unroll
+      for (int q = 0; q < E / R0; q++)
+#pragma unroll
+        for (int r = 0; r < R0; r++) val[q * R0 + r] = fetch(s, t + q * P + r * (N / R0));
+    }
 #pragma unroll
     for (int q = 0; q < E / R0; q++)
 #pragma unroll
@@ -468,7 +487,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
 }
 
 // ---------------------------------------------------------------------------
-// K3: x-line chain.  grid (nzt, n): one block = TZ x-lines (z = zt*TZ + zz)
+// K3: x-line chain.  grid (n / TZ, n): one block = TZ x-lines (k3_tz) (z = zt*TZ + zz)
 // at one y.  Two real lines are carried in one complex FFT (pairs zz=2p,2p+1).
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -479,12 +498,12 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* addr, double 
 // The z-pencil slots of a K3 tile: pair p of tile zt is the real lines z =
 // zt TZ + 2 p and the next one; element x of the first sits at element
 // off(x) of its plane, the second's BS elements on.
-template <typename T, int N> struct XPair {
+template <typename T, int N, int TZ> struct XPair {
   using PA = Panel<T, N>;
   static constexpr int BS = PA::DBL ? PA::ROW : 1;
   unsigned row, s;   // element of the pair's row in a panel, slot rotation
   __device__ __forceinline__ XPair(int zt, int p) {
-    const unsigned rho = (unsigned)(zt * Tiles<T>::TZ + 2 * p) / PA::ZS;
+    const unsigned rho = (unsigned)(zt * TZ + 2 * p) / PA::ZS;
     row = rho * PA::ROW;
     s = PA::sw(rho);
   }
@@ -500,16 +519,16 @@ template <typename T, int N> struct XPair {
   }
 };
 
-template <typename T, int N>
+template <typename T, int N, int TZ>
 __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int nbuf, int L,
                                              C2<T>* __restrict__ uz, int slot0, int y, int zt,
                                              T half_factor) {
   using C = C2<T>;
-  constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
+  constexpr int NPAIR = TZ / 2;
   const int kxn = g.kxn;
   // thread -> fixed pair p, x strided by blockDim/NPAIR (no runtime division)
   const int p = threadIdx.x % NPAIR, x0 = threadIdx.x / NPAIR, xs = blockDim.x / NPAIR;
-  const XPair<T, N> xp(zt, p);
+  const XPair<T, N, TZ> xp(zt, p);
   for (int b = 0; b < nbuf; b++)
   for (int x = x0; x < kxn; x += xs) {
     const C* line = buf + (b * NPAIR + p) * L;
@@ -519,7 +538,7 @@ __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int
     const C B = cmk<C>((Y.y + Yn.y) * half_factor, (Yn.x - Y.x) * half_factor);
     C* dst = uz + ((size_t)(slot0 + b) * N + y) * uz_slab<T>(N) + xp.off(x);
     dst[0] = A;
-    dst[XPair<T, N>::BS] = B;
+    dst[XPair<T, N, TZ>::BS] = B;
   }
 }
 
@@ -528,16 +547,16 @@ __device__ __forceinline__ void xchain_store(const Geo& g, const C2<T>* buf, int
 // extension and the imaginary part of the kx=0 term dropped; stored
 // conjugated (backward transform by conjugation).  All loads of a thread are
 // issued before the first shared-memory store.
-template <typename T, int N, int NV, int THREADS>
+template <typename T, int N, int NV, int THREADS, int TZ>
 __device__ __forceinline__ void xchain_pack(const Geo& g, const C2<T>* __restrict__ uz, int v0, int y, int zt,
                                             C2<T>* bufU, int L) {
   using C = C2<T>;
-  constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
+  constexpr int NPAIR = TZ / 2;
   constexpr int XST = THREADS / NPAIR;
   constexpr int XI = (N / 2 + XST - 1) / XST;
   const int kxn = g.kxn;
   const int p = threadIdx.x % NPAIR, xth = threadIdx.x / NPAIR;
-  const XPair<T, N> xp(zt, p);
+  const XPair<T, N, TZ> xp(zt, p);
   C A[NV][XI], B[NV][XI];
 #pragma unroll
   for (int v = 0; v < NV; v++)
@@ -552,7 +571,7 @@ __device__ __forceinline__ void xchain_pack(const Geo& g, const C2<T>* __restric
           B[v][i] = cmk<C>(q.z, q.w);
         } else {
           A[v][i] = src[0];
-          B[v][i] = src[XPair<T, N>::BS];
+          B[v][i] = src[XPair<T, N, TZ>::BS];
         }
       }
     }
@@ -595,13 +614,13 @@ struct XFuse {
 // band kx in [kxn, N - kxn] zero), and pass 0's output goes to shared memory.
 // Every thread of the block runs the same rounds (the shuffles name whole
 // warps); loads and stores are predicated on the line being one of NV NPAIR.
-template <typename T, int N, int NV, int THREADS>
+template <typename T, int N, int NV, int THREADS, int TZ>
 __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __restrict__ uz, int v0, int y,
                                                   int zt, C2<T>* buf, int L) {
   using C = C2<T>;
   using PL = FFTPlan<T, N>;
   static_assert(XFuse<T, N>::value, "plan without register-level packing");
-  constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
+  constexpr int NPAIR = TZ / 2;
   constexpr int R0 = PL::rad(0), R1 = PL::rad(1), P = PL::P, E = PL::E, H = R1 / 2;
   constexpr int LPR = THREADS / P, NB = E / R0;
   static_assert(THREADS % 32 == 0, "whole warps");
@@ -612,7 +631,7 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
     const int l = l0 + lr;
     const bool act = l < NV * NPAIR;
     const int v = act ? l / NPAIR : 0, p = l % NPAIR;
-    const XPair<T, N> xp(zt, p);
+    const XPair<T, N, TZ> xp(zt, p);
     const C* col = uz + ((size_t)(v0 + v) * N + y) * uz_slab<T>(N);
     const size_t o0 = xp.off(t);
     C a[H], b[H];
@@ -628,7 +647,7 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
           b[m] = cmk<C>(q.z, q.w);
         } else {
           a[m] = col[xp.off(o0, t, m)];
-          b[m] = col[xp.off(o0, t, m) + XPair<T, N>::BS];
+          b[m] = col[xp.off(o0, t, m) + XPair<T, N, TZ>::BS];
         }
       }
     }
@@ -670,14 +689,14 @@ __device__ __forceinline__ void xchain_load_pass0(const Geo& g, const C2<T>* __r
 // unpacking done in registers: A(x), B(x) of the real lines z = zt TZ + 2p,
 // 2p + 1 go to uz slot l / NPAIR for x < kxn.  Called by every thread of
 // the block (whole warps per round).
-template <typename T, int N, int THREADS>
+template <typename T, int N, int THREADS, int TZ>
 __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf, int nlines, int L,
                                                   const C2<T>* tw, C2<T>* __restrict__ uz, int y, int zt,
                                                   T half_factor) {
   using C = C2<T>;
   using PL = FFTPlan<T, N>;
   static_assert(XFuse<T, N>::value, "plan without register-level packing");
-  constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
+  constexpr int NPAIR = TZ / 2;
   constexpr int R1 = PL::rad(1), P = PL::P, E = PL::E, H = R1 / 2, NS = PL::ns(1);
   constexpr int LPR = THREADS / P;
   static_assert(NS == P && E == R1, "the last pass holds elements t + P m");
@@ -695,7 +714,7 @@ __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf
       for (int m = 0; m < E; m++) v[m] = cmk<C>(0, 0);
     }
     const int b = act ? l / NPAIR : 0, p = l % NPAIR;
-    const XPair<T, N> xp(zt, p);
+    const XPair<T, N, TZ> xp(zt, p);
     C* col = uz + ((size_t)b * N + y) * uz_slab<T>(N);
     const size_t o0 = xp.off(t);
 #pragma unroll
@@ -712,26 +731,35 @@ __device__ __forceinline__ void xchain_last_store(const Geo& g, const C2<T>* buf
           *reinterpret_cast<float4*>(col + xp.off(o0, t, m)) = make_float4(ax, ay, bx, by);
         } else {
           col[xp.off(o0, t, m)] = cmk<C>(ax, ay);
-          col[xp.off(o0, t, m) + XPair<T, N>::BS] = cmk<C>(bx, by);
+          col[xp.off(o0, t, m) + XPair<T, N, TZ>::BS] = cmk<C>(bx, by);
         }
       }
     }
   }
 }
 
-// K3 runs the five output products of a tile as one batch of 5 * TZ/2
-// lines: one warp per line at n = 1024 (a multiple of 32 threads, so that
-// the velmax warp reduction sees whole warps)
-template <typename T, int N, int NC>
+// z lines of a K3 tile (dbl: FP64 state; nf fields in a batch): one pair where
+// its lines fill whole warps (small blocks overlap their phases better: 1024^3
+// FP32 8.86 ms with two pairs in blocks of ten warps, 8.53 with one in five;
+// 512^3 with a scalar 1.74 and 1.45 ms), else two in FP32 (512^3, 5 lines of 16
+// threads: 1.01 ms with two pairs, 1.17 with one).
+__host__ __device__ constexpr int k3_tz(bool dbl, int n, int nf, bool tcm) {
+  return dbl || (!tcm && nf * (n / plan_e(n, false)) % 32 == 0) ? 2 : 4;
+}
+
+// K3 runs the output products of a tile as one batch of (5 + NC) TZ/2 lines:
+// one warp per line at n = 1024 (a multiple of 32 threads, so that the velmax
+// warp reduction sees whole warps)
+template <typename T, int N, int NC, bool TCM = false>
 struct K3Launch {
   static constexpr int P = FFTPlan<T, N>::P;
-  static constexpr int NPAIR = Tiles<T>::TZ / 2;
-  static constexpr int want = 5 * NPAIR * P;
+  static constexpr int TZ = k3_tz(sizeof(T) == 8, N, 5 + NC, TCM), NPAIR = TZ / 2;
+  static constexpr int want = (5 + NC) * NPAIR * P;
   static constexpr int WP = 32 / gcd_c(32, P) * P;   // lcm(32, P): whole warps and whole lines
   static constexpr int THREADS = round_up(want, WP) > 1024 ? 1024 : round_up(want, WP);
   static_assert(THREADS % P == 0, "threads per line must divide the block");
   // registers sized for twenty warps per SM (about 100 a thread)
-  static constexpr int MINB = 640 / THREADS < 2 ? 2 : (640 / THREADS > 10 ? 10 : 640 / THREADS);
+  static constexpr int MINB = TCM ? 1 : (640 / THREADS < 2 ? 2 : (640 / THREADS > 10 ? 10 : 640 / THREADS));
   // twiddles + 5 product buffers (6 input buffers with a scalar) of TZ/2 lines
   static constexpr size_t SMEM =
       sizeof(C2<T>) * (FFTPlan<T, N>::TWSIZE + (size_t)(NC ? 6 : 5) * NPAIR * LS<T, N>::value);
@@ -761,7 +789,7 @@ __device__ __forceinline__ void velmax_point(C U, C V, C W, double xn, double yn
 }
 
 template <typename T, int N, int NC = 0, bool TCM = false>
-__global__ void __launch_bounds__(K3Launch<T, N, NC>::THREADS, TCM ? 1 : K3Launch<T, N, NC>::MINB)
+__global__ void __launch_bounds__(K3Launch<T, N, NC, TCM>::THREADS, K3Launch<T, N, NC, TCM>::MINB)
 k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T b22, T b33,
          unsigned long long* velmax_bits, int want_velmax, T cb1 = T(0), T cb2 = T(0), T cb3 = T(0),
          TcArgs tca = TcArgs()) {
@@ -769,9 +797,10 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   // 5 = d/dz); the advection term u.(G + grad theta) (itransform.f:522-530,
   // G = cb, init.f:42-45) is formed in physical space and goes to slot 5.
   using C = C2<T>;
-  constexpr int TZ = Tiles<T>::TZ, NPAIR = TZ / 2;
+  using KL = K3Launch<T, N, NC, TCM>;
+  constexpr int TZ = KL::TZ, NPAIR = TZ / 2;
   constexpr int NVIN = 3 + 3 * NC;
-  constexpr int THREADS = K3Launch<T, N, NC>::THREADS;
+  constexpr int THREADS = KL::THREADS;
   constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
@@ -782,11 +811,11 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   C* bufE = bufW + NPAIR * L;
   C* bufF = bufE + NPAIR * L;
   load_twiddles<T, N>(tw, tw_g);
-  constexpr int NCOL = tc_cols(K3Launch<T, N, NC>::LINES_TC);
+  constexpr int NCOL = tc_cols(KL::LINES_TC);
   tc::Work w;
   if constexpr (TCM)
-    tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(bufU + K3Launch<T, N, NC>::LINES_TC * L), tca);
-  // grid (nzt, n, boxes)
+    tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(bufU + KL::LINES_TC * L), tca);
+  // grid (n / TZ, n, boxes)
   const int zt = blockIdx.x, y = blockIdx.y, box = blockIdx.z;
   uz += box * g.zbox;
   velmax_bits += box;
@@ -795,7 +824,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   // tensor-core path and the other plans go through shared memory
   constexpr bool FUSE = !TCM && XFuse<T, N>::value;
   if constexpr (FUSE) {
-    xchain_load_pass0<T, N, NVIN, THREADS>(g, uz, 0, y, zt, bufU, L);
+    xchain_load_pass0<T, N, NVIN, THREADS, TZ>(g, uz, 0, y, zt, bufU, L);
     cp_async_wait_all();
     __syncthreads();
     fft_passes<T, N, THREADS, 1>(bufU, NVIN * NPAIR, L, tw);
@@ -806,8 +835,8 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
       const int k = e % N;
       if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
     }
-    xchain_pack<T, N, 3, THREADS>(g, uz, 0, y, zt, bufU, L);
-    if constexpr (NC > 0) xchain_pack<T, N, 3, THREADS>(g, uz, 3, y, zt, bufU + 3 * NPAIR * L, L);
+    xchain_pack<T, N, 3, THREADS, TZ>(g, uz, 0, y, zt, bufU, L);
+    if constexpr (NC > 0) xchain_pack<T, N, 3, THREADS, TZ>(g, uz, 3, y, zt, bufU + 3 * NPAIR * L, L);
     cp_async_wait_all();
     __syncthreads();
     lines_fft<T, N, THREADS, TCM>(bufU, NVIN * NPAIR, L, tw, w);
@@ -853,11 +882,11 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
     // pass 0 in shared memory; each line's last pass runs on the warp that
     // wrote it, so a warp barrier (inside fft_pass) orders the two
     fft_passes_until<T, N, THREADS, 0, 1>(bufU, (5 + NC) * NPAIR, L, tw);
-    xchain_last_store<T, N, THREADS>(g, bufU, (5 + NC) * NPAIR, L, tw, uz, y, zt, hf);
+    xchain_last_store<T, N, THREADS, TZ>(g, bufU, (5 + NC) * NPAIR, L, tw, uz, y, zt, hf);
   } else {
     lines_fft<T, N, THREADS, TCM>(bufU, (5 + NC) * NPAIR, L, tw, w);
     if constexpr (TCM) tc::teardown<NCOL>(w);
-    xchain_store<T, N>(g, bufU, 5 + NC, L, uz, 0, y, zt, hf);
+    xchain_store<T, N, TZ>(g, bufU, 5 + NC, L, uz, 0, y, zt, hf);
   }
 }
 
@@ -1075,7 +1104,7 @@ k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>*
   // NC = 1: the scalar advection term (uz slot 5) goes to ub slot 4 without
   // derivatives (transform.f: i2f = 4+nc)
   using C = C2<T>;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   if constexpr (!TCM) {
     zfwd_panels<T, N, NC, PPBO>(g, uz, ub, smem_raw, tw_g, ntiles, b11, b33);
   } else {
@@ -1413,7 +1442,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
   const int zt = blockIdx.x, y = blockIdx.y;
   const int kxn = g.kxn;
   if constexpr (XFuse<T, N>::value) {
-    xchain_load_pass0<T, N, 3, THREADS>(g, uz, 0, y, zt, bufU, L);
+    xchain_load_pass0<T, N, 3, THREADS, TZ>(g, uz, 0, y, zt, bufU, L);
     cp_async_wait_all();
     __syncthreads();
     fft_passes<T, N, THREADS, 1>(bufU, 3 * NPAIR, L, tw);
@@ -1423,7 +1452,7 @@ k_xspline(Geo g, const C2<T>* __restrict__ uz, typename V4T<T>::type* __restrict
       const int k = e % N;
       if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
     }
-    xchain_pack<T, N, 3, THREADS>(g, uz, 0, y, zt, bufU, L);
+    xchain_pack<T, N, 3, THREADS, TZ>(g, uz, 0, y, zt, bufU, L);
     cp_async_wait_all();
     __syncthreads();
     fft_lines<T, N, THREADS>(bufU, 3 * NPAIR, L, tw);
@@ -1470,7 +1499,7 @@ k_xmoments(Geo g, const C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, 
     const int k = e % N;
     if (k >= kxn && k <= N - kxn) bufU[(e / N) * L + padl<C, N>(k)] = cmk<C>(0, 0);
   }
-  xchain_pack<T, N, 2, THREADS>(g, uz, 0, y, zt, bufU, L);
+  xchain_pack<T, N, 2, THREADS, TZ>(g, uz, 0, y, zt, bufU, L);
   cp_async_wait_all();
   __syncthreads();
   fft_lines<T, N, THREADS>(bufU, 2 * NPAIR, L, tw);

@@ -195,7 +195,7 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   k_zinv<T, N><<<dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st>>>(geo, ub, uz, twd);
   {
     constexpr int TH = K3Launch<T, N, 0>::THREADS;
-    k_xchain<T, N><<<dim3(geo.nzt, N), TH, K3Launch<T, N, 0>::SMEM, st>>>(
+    k_xchain<T, N><<<dim3(N / K3Launch<T, N, 0>::TZ, N), TH, K3Launch<T, N, 0>::SMEM, st>>>(
         geo, uz, twd, stb.b11, stb.b22, stb.b33, vmx, kstep == 1 ? 1 : 0);
   }
   const int tiles = N * ZL::TILES;
