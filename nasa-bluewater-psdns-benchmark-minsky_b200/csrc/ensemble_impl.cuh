@@ -158,9 +158,9 @@ template <typename T, int N> struct EnsImpl {
     C* u = (C*)e.d_u + (size_t)b0 * e.st_elems;
     C* un = (C*)e.d_un + (size_t)b0 * e.st_elems;
     if (kstep == 1)
-      k_yfwd<T, N, 1><<<dim3(e.nab_f, nb), TH, I::sm5(), e.stream>>>(g, st, ub, u, un, (const C*)e.d_tw, nullptr);
+      k_yfwd<T, N, 1><<<dim3(K5Launch<T, N, 0>::blocks(e.nab_f), nb), TH, I::sm5(), e.stream>>>(g, st, ub, u, un, (const C*)e.d_tw, nullptr);
     else
-      k_yfwd<T, N, 2><<<dim3(e.nab_f, nb), TH, I::sm5(), e.stream>>>(g, st, ub, u, un, (const C*)e.d_tw, nullptr);
+      k_yfwd<T, N, 2><<<dim3(K5Launch<T, N, 0>::blocks(e.nab_f), nb), TH, I::sm5(), e.stream>>>(g, st, ub, u, un, (const C*)e.d_tw, nullptr);
     CK(cudaGetLastError());
     return 0;
   }

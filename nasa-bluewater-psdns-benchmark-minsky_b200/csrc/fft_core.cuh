@@ -532,26 +532,34 @@ __device__ __forceinline__ void fft_passes_until(C2<T>* buf, int nlines, int ls,
 // xor a constant, and the constant's bits above the permuted ones go into the
 // instruction's immediate offset.
 // ---------------------------------------------------------------------------
-template <typename T, int N> struct Panel {
+// SLOT1: the y transforms' panel of one slot a row (two FP32 columns side by
+// side, one FP64 column), 16 N bytes; the columns of a slot swap with bit 3 of
+// the row for the same reason.
+template <typename T_, int N_, bool SLOT1 = false> struct Panel {
+  using T = T_;
+  static constexpr int N = N_;
   using C = C2<T>;
   using PL = FFTPlan<T, N>;
   static constexpr bool DBL = sizeof(T) == 8, POW2 = is_pow2(N);
-  static constexpr int ZS = DBL ? 1 : 2, PW = DBL ? 4 : 8;
+  static constexpr int ZS = SLOT1 || DBL ? 1 : 2, PW = SLOT1 ? (DBL ? 1 : 2) : (DBL ? 4 : 8);
+  static constexpr unsigned LX = SLOT1 ? 8 : 16;   // line x: xor LX x (SLOT1: FP32 only)
   static constexpr int ROW = PW * ZS;            // complex elements of a row
   static constexpr int ELEMS = N * PW;           // of a panel
   static constexpr unsigned BYTES = ELEMS * sizeof(C);
-  static constexpr unsigned LOW = DBL ? 511 : 1023;   // bytes that the orders permute within
+  static constexpr unsigned LOW = SLOT1 ? 255 : DBL ? 511 : 1023;   // bytes that the orders permute within
   static constexpr int S = POW2 ? ilog2c(PL::rad(0)) : 0;
   static constexpr unsigned M = !POW2 ? 0 : (PL::rad(0) < (DBL ? 8 : 16) ? PL::rad(0) : (DBL ? 8 : 16)) - 1;
-  static_assert(N % ZS == 0 && BYTES % 1024 == 0, "panels keep the alignment that xor addressing needs");
-  __host__ __device__ static constexpr unsigned sw(unsigned rho) { return DBL ? (rho >> 1) & 3 : rho & 7; }
-  // byte offset of element i of line 0 (line x: xor 16 x)
+  static_assert(N % ZS == 0 && BYTES % (LOW + 1) == 0, "panels keep the alignment that xor addressing needs");
+  __host__ __device__ static constexpr unsigned sw(unsigned rho) {
+    return SLOT1 ? (DBL ? 0 : (rho >> 3) & 1) : DBL ? (rho >> 1) & 3 : rho & 7;
+  }
+  // byte offset of element i of line 0 (line x: xor LX x)
   template <bool XCH> __host__ __device__ static constexpr unsigned off(unsigned i) {
     if (XCH) i ^= (i >> S) & M;
     const unsigned rho = i / ZS;
-    return rho * (ROW * sizeof(C)) + sw(rho) * 16 + (i % ZS) * sizeof(C);
+    return rho * (ROW * sizeof(C)) + sw(rho) * LX + (i % ZS) * sizeof(C);
   }
-  // element a + B of the line at byte offset o (panel offset + 16 x); the bits
+  // element a + B of the line at byte offset o (panel offset + LX x); the bits
   // of a and B are disjoint for N = 2^k
   template <bool XCH, unsigned B> __device__ __forceinline__ static C& at(unsigned char* smem, unsigned oa, unsigned o, unsigned a) {
     if constexpr (POW2) {
@@ -563,40 +571,38 @@ template <typename T, int N> struct Panel {
   }
 };
 
-template <typename T, int N, bool XCH, int R, int STEP, int r = 0>
-__device__ __forceinline__ void panel_read(unsigned char* smem, unsigned oa, unsigned o, unsigned a, C2<T>* v) {
+template <typename PA, bool XCH, int R, int STEP, int r = 0>
+__device__ __forceinline__ void panel_read(unsigned char* smem, unsigned oa, unsigned o, unsigned a, typename PA::C* v) {
   if constexpr (r < R) {
-    v[r] = Panel<T, N>::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a);
-    panel_read<T, N, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
+    v[r] = PA::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a);
+    panel_read<PA, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
   }
 }
-template <typename T, int N, bool XCH, int R, int STEP, int r = 0>
-__device__ __forceinline__ void panel_write(unsigned char* smem, unsigned oa, unsigned o, unsigned a, const C2<T>* v) {
+template <typename PA, bool XCH, int R, int STEP, int r = 0>
+__device__ __forceinline__ void panel_write(unsigned char* smem, unsigned oa, unsigned o, unsigned a, const typename PA::C* v) {
   if constexpr (r < R) {
-    Panel<T, N>::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a) = v[r];
-    panel_write<T, N, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
+    PA::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a) = v[r];
+    panel_write<PA, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
   }
 }
 
 // elements t + q P + r (N / R) of a line, natural order (r < R, q < E / R)
-template <typename T, int N, int R>
-__device__ __forceinline__ void panel_load(unsigned char* smem, unsigned o, int t, C2<T>* v) {
-  using PA = Panel<T, N>;
-  using PL = FFTPlan<T, N>;
+template <typename PA, int R>
+__device__ __forceinline__ void panel_load(unsigned char* smem, unsigned o, int t, typename PA::C* v) {
+  using PL = typename PA::PL;
 #pragma unroll
   for (int q = 0; q < PL::E / R; q++) {
     const unsigned a = t + q * PL::P;
-    panel_read<T, N, false, R, N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
+    panel_read<PA, false, R, PA::N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
   }
 }
-template <typename T, int N, int R>
-__device__ __forceinline__ void panel_store(unsigned char* smem, unsigned o, int t, const C2<T>* v) {
-  using PA = Panel<T, N>;
-  using PL = FFTPlan<T, N>;
+template <typename PA, int R>
+__device__ __forceinline__ void panel_store(unsigned char* smem, unsigned o, int t, const typename PA::C* v) {
+  using PL = typename PA::PL;
 #pragma unroll
   for (int q = 0; q < PL::E / R; q++) {
     const unsigned a = t + q * PL::P;
-    panel_write<T, N, false, R, N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
+    panel_write<PA, false, R, PA::N / R>(smem, o ^ PA::template off<false>(a), o, a, v + q * R);
   }
 }
 
@@ -605,18 +611,17 @@ __device__ __forceinline__ void panel_store(unsigned char* smem, unsigned o, int
 // v[q R0 + r]) in, the outputs of the last pass (element t + q P + r NS in
 // v[q R + r]) out; afterwards every slot of the line has been read.  Called by
 // whole warps.
-template <typename T, int N, bool INV>
-__device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t, const C2<T>* tw, C2<T>* v) {
-  using PA = Panel<T, N>;
-  using PL = FFTPlan<T, N>;
+template <typename PA, bool INV>
+__device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t, const typename PA::C* tw, typename PA::C* v) {
+  using PL = typename PA::PL;
   static_assert(PL::NPASS >= 2, "load and store passes must differ");
-  constexpr int E = PL::E, P = PL::P, R0 = PL::rad(0);
+  constexpr int N = PA::N, E = PL::E, P = PL::P, R0 = PL::rad(0);
 #pragma unroll
   for (int q = 0; q < E / R0; q++) dft_s<R0, 1, INV>(v + q * R0);
 #pragma unroll
   for (int q = 0; q < E / R0; q++) {
     const unsigned a = (t + q * P) * R0;
-    panel_write<T, N, true, R0, 1>(smem, o ^ PA::template off<true>(a), o, a, v + q * R0);
+    panel_write<PA, true, R0, 1>(smem, o ^ PA::template off<true>(a), o, a, v + q * R0);
   }
   line_sync<P>();
   if constexpr (PL::NPASS == 3) {
@@ -624,7 +629,7 @@ __device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t
 #pragma unroll
     for (int q = 0; q < E / R; q++) {
       const unsigned a = t + q * P;
-      panel_read<T, N, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+      panel_read<PA, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
     }
     line_sync<P>();
 #pragma unroll
@@ -632,7 +637,7 @@ __device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t
       const int j = t + q * P;
       dft_tw<R, NS, INV>(v + q * R, tw + PL::twoff(1) + j % NS);
       const unsigned a = (j / NS) * NS * R + j % NS;
-      panel_write<T, N, true, R, NS>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+      panel_write<PA, true, R, NS>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
     }
     line_sync<P>();
   }
@@ -640,7 +645,7 @@ __device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t
 #pragma unroll
   for (int q = 0; q < E / R; q++) {
     const unsigned a = t + q * P;
-    panel_read<T, N, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
+    panel_read<PA, true, R, N / R>(smem, o ^ PA::template off<true>(a), o, a, v + q * R);
   }
   line_sync<P>();
 #pragma unroll

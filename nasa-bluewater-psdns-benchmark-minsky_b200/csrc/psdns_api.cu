@@ -336,7 +336,8 @@ template <typename T, int N, int NC> struct Impl {
   static size_t sm2() { return ZL::SMEM2; }
   static size_t sm3() { return K3Launch<T, N, NC>::SMEM; }
   static size_t sm4() { return ZL::SMEM4; }
-  static size_t sm5() { return TWB + sizeof(C) * (4 + NC) * TL::TB_F * L; }
+  static size_t sm5() { return K5Launch<T, N, NC>::SMEM; }
+  static size_t sm5tc() { return K5Launch<T, N, NC>::SMEM_TC; }
   static size_t sm1tc() { return TWB + sizeof(C) * TL::TB_I * L + kTcTail; }
   static size_t sm2tc() { return TWB + sizeof(C) * kTcXT2 * L + kTcTail; }
   static size_t sm4tc() { return TWB + sizeof(C) * 2 * kTcXT4 * L + kTcTail; }
@@ -362,9 +363,9 @@ template <typename T, int N, int NC> struct Impl {
       CK(cudaFuncSetAttribute(k_zfwd<T, N, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)sm4tc()));
       CK(cudaFuncSetAttribute(k_yfwd<T, N, 1, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sm5() + kTcTail)));
+                              (int)sm5tc()));
       CK(cudaFuncSetAttribute(k_yfwd<T, N, 2, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(sm5() + kTcTail)));
+                              (int)sm5tc()));
     }
     CK(cudaFuncSetAttribute(k_yinv<T, N, false, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1()));
     CK(cudaFuncSetAttribute(k_zinv<T, N, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2()));
@@ -479,7 +480,7 @@ template <typename T, int N, int NC> struct Impl {
       double* d_tk = (double*)c.d_efkz;   // n/2 + 2 shells of 3 doubles: room for n/2
       if (cudaMemsetAsync(d_tk, 0, sizeof(double) * (N / 2), c.stream) != cudaSuccess) rc = set_error("memset");
       if (!rc) {
-        k_yfwd<T, N, 0, NC><<<c.nab_f, K5Launch<T, N, NC>::THREADS, sm5() + sizeof(double) * (N / 2), c.stream>>>(
+        k_yfwd<T, N, 0, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), K5Launch<T, N, NC>::THREADS, sm5() + sizeof(double) * (N / 2), c.stream>>>(
             g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, d_tk);
         if (cudaGetLastError() != cudaSuccess) rc = set_error("transfer launch failed");
       }
@@ -588,13 +589,13 @@ template <typename T, int N, int NC> struct Impl {
     Geo g = make_geo(c);
     StageTables<T> st = make_tables<T>(c, (kstep - 1) & 1);
     const TcArgs ta = tc_args(c);
-    constexpr int TH = K5Launch<T, N, NC>::THREADS;
+    constexpr int TH = K5Launch<T, N, NC>::THREADS_TC;
     prof_mark(c, kstep - 1, 4, 0);
     if (kstep == 1)
-      k_yfwd<T, N, 1, NC, true><<<c.nab_f, TH, sm5() + kTcTail, c.stream>>>(
+      k_yfwd<T, N, 1, NC, true><<<c.nab_f, TH, sm5tc(), c.stream>>>(
           g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, ta);
     else
-      k_yfwd<T, N, 2, NC, true><<<c.nab_f, TH, sm5() + kTcTail, c.stream>>>(
+      k_yfwd<T, N, 2, NC, true><<<c.nab_f, TH, sm5tc(), c.stream>>>(
           g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, ta);
     prof_mark(c, kstep - 1, 4, 1);
     CK(cudaGetLastError());
@@ -613,10 +614,10 @@ template <typename T, int N, int NC> struct Impl {
       const C* tw = (const C*)c.d_tw;
       prof_mark(c, kstep - 1, 4, 0);
       switch (kstep) {
-        case 1: k_yfwd<T, N, 11><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 2: k_yfwd<T, N, 12><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 3: k_yfwd<T, N, 13><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        default: k_yfwd<T, N, 14><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r);
+        case 1: k_yfwd<T, N, 11><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        case 2: k_yfwd<T, N, 12><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        case 3: k_yfwd<T, N, 13><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        default: k_yfwd<T, N, 14><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r);
       }
       prof_mark(c, kstep - 1, 4, 1);
       CK(cudaGetLastError());
@@ -635,10 +636,10 @@ template <typename T, int N, int NC> struct Impl {
     constexpr int TH = K5Launch<T, N, NC>::THREADS;
     prof_mark(c, kstep - 1, 4, 0);
     if (kstep == 1)
-      k_yfwd<T, N, 1, NC><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
+      k_yfwd<T, N, 1, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
                                                         (const C*)c.d_tw, c.d_efkz);
     else
-      k_yfwd<T, N, 2, NC><<<c.nab_f, TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
+      k_yfwd<T, N, 2, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
                                                         (const C*)c.d_tw, c.d_efkz);
     prof_mark(c, kstep - 1, 4, 1);
     CK(cudaGetLastError());

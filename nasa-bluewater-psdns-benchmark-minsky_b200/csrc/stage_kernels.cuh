@@ -3,7 +3,9 @@
 // Device data layout (one box, n^3, kxn kx columns, xz_tot cylinder columns):
 //   u, un  [v][a][y]                 y-cylinders, the reference's uy(ny,num_al,v)
 //   ub     [v][a/TB][y][a%TB]         cylinder data with y and a swapped in
-//                                    blocks of TB columns (TB_I inverse, TB_F forward)
+//                                    blocks of TB columns (TBL_I inverse, TBL_F forward;
+//                                    forward FP32: the columns of a pair swap with bit 3
+//                                    of y, ubf_swap)
 //   uz     [v][y][x/PW] panels        z-pencils for x < kxn (rounded up to panels of PW
 //                                    lines): Panel of fft_core.cuh, rows of one z slot
 // Per stage:
@@ -110,19 +112,24 @@ template <typename T> struct StageTables {
 // K2's reads), filled by pairs of K1 blocks.
 template <typename T> struct Tiles;
 template <> struct Tiles<float> {
-  static constexpr int TB_I = 8, TBL_I = 16, TB_F = 4, TBL_F = 8, TZ = 4;
+  static constexpr int TB_I = 8, TBL_I = 16, TB_F = 2, TBL_F = 8, TZ = 4;
 };
 template <> struct Tiles<double> {
-  static constexpr int TB_I = 4, TBL_I = 8, TB_F = 2, TBL_F = 4, TZ = 2;
+  static constexpr int TB_I = 4, TBL_I = 8, TB_F = 1, TBL_F = 4, TZ = 2;
 };
 
 // elements of one variable of the forward ub layout [a/TBL_F][y][a%TBL_F]
-// (K4 writes 64-byte runs; K5 blocks of TB_F columns read halves)
+// (K4 writes 64-byte runs; K5 blocks of TB_F columns read 16-byte quarters)
 template <typename T>
 __host__ __device__ __forceinline__ size_t ubf_var_elems(int nab_f, int n) {
   constexpr int R = Tiles<T>::TBL_F / Tiles<T>::TB_F;
   return (size_t)((nab_f + R - 1) / R * R) * Tiles<T>::TB_F * n;
 }
+
+// what column a of the forward ub layout is xored with at row y: the order of
+// the y transforms' shared-memory panels (Panel with SLOT1)
+template <typename T>
+__device__ __forceinline__ int ubf_swap(int y) { return sizeof(T) == 4 ? (y >> 3) & 1 : 0; }
 
 // elements of one variable of the inverse ub layout [a/TBL_I][y][a%TBL_I]
 template <typename T>
@@ -217,10 +224,37 @@ struct ZLaunch {
   static constexpr int MINB4 = resident_blocks(SMEM4, THREADS, 16);
 };
 
-// K5 holds one CTA per SM (its (4 + nc) * TB_F lines fill shared memory), so
-// it runs every line of a block at once
+// K5: the lines of a block's columns (4 + nc fields) at once, a group of P
+// threads each.  SLOT, n >= 512: one slot of TB_F columns in one-slot panels (64
+// KB at n = 1024: three blocks per SM where four FP32 columns in padded lines
+// held one; FP32 8.67 -> 7.67 ms, FP64 19.1 -> 15.6; 512^3 1.00 -> 0.89 and
+// 2.72 -> 1.80).  Smaller n: two slots in padded lines, which keep more blocks
+// resident anyway and whose copies take whole sectors (256^3 FP32 0.108 ms
+// against 0.114 with panels, 96^3 with a scalar 16.4 us against 19.9).
+constexpr size_t kTcTailBytes = tc::kBBytes + 16;
 template <typename T, int N, int NC>
-struct K5Launch : Launch<T, N, (4 + NC) * Tiles<T>::TB_F, 1024> {};
+struct K5Launch {
+  using PA = Panel<T, N, true>;
+  static_assert(PA::PW == Tiles<T>::TB_F, "a panel holds one slot's columns");
+  static constexpr bool SLOT = N >= 512;
+  static constexpr int SPB = SLOT ? 1 : 2, COLS = SPB * Tiles<T>::TB_F;
+  static constexpr int P = FFTPlan<T, N>::P, LINES = (4 + NC) * COLS;
+  static constexpr int blocks(int nslots) { return (nslots + SPB - 1) / SPB; }
+  static constexpr int THREADS = Launch<T, N, LINES, 1024>::THREADS;
+  static_assert(!SLOT || THREADS == LINES * P, "a group per line");
+  static constexpr size_t TWB = sizeof(C2<T>) * FFTPlan<T, N>::TWSIZE;
+  static constexpr size_t SMEM =
+      TWB + (SLOT ? (size_t)(4 + NC) * PA::BYTES : sizeof(C2<T>) * LINES * LS<T, N>::value);
+  // registers sized for 24 warps per SM in FP32 and with the short FP64 operand
+  // lists of n = 512, sixteen or twelve with longer ones: left to itself the
+  // compiler takes up to 136 in FP32 and a block less fits (256^3 with a scalar
+  // 0.204 ms against 0.157)
+  static constexpr int WARPS = sizeof(T) == 4 || FFTPlan<T, N>::E <= 8 ? 24 : (SLOT ? 16 : 12);
+  static constexpr int MINB = resident_blocks(SMEM, round_up(THREADS, 32), WARPS);
+  // tensor-core form: one slot in padded lines
+  static constexpr int LINES_TC = (4 + NC) * Tiles<T>::TB_F, THREADS_TC = Launch<T, N, LINES_TC, 1024>::THREADS;
+  static constexpr size_t SMEM_TC = TWB + sizeof(C2<T>) * LINES_TC * LS<T, N>::value + kTcTailBytes;
+};
 
 // Mixed-precision form of the stage kernels (template flag TCM, FP32 state
 // at n = 1024): every 1024-point transform runs on the tensor cores
@@ -233,7 +267,7 @@ struct TcArgs {
   const float2* tw2 = nullptr;
   unsigned* err = nullptr;
 };
-constexpr size_t kTcTail = tc::kBBytes + 16;
+constexpr size_t kTcTail = kTcTailBytes;
 // z tiles of the tensor-core kernels, independent of Tiles<float>: an operand
 // tile (32 KB) overlays four lines, so every line buffer that one transform
 // call runs on holds at least four lines
@@ -468,8 +502,8 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
     cp_async_wait_all();
     __syncthreads();   // the twiddles
     const unsigned o = (l / PA::PW) * PA::BYTES + (l % PA::PW) * 16;
-    panel_fft<T, N, true>(smem_raw, o, t, tw, val);
-    panel_store<T, N, RL>(smem_raw, o, t, val);
+    panel_fft<PA, true>(smem_raw, o, t, tw, val);
+    panel_store<PA, RL>(smem_raw, o, t, val);
     // every thread's writes before the copy engine's reads
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
@@ -916,6 +950,7 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
   const int as = abeg - (abeg % TB);                      // first block boundary
   const int cnt = ((aend - as + TB - 1) / TB) * TB;  // whole blocks
   C* dst = ub + (size_t)slot * ubf_var_elems<T>(g.nab_f, N);
+  const int swap = ubf_swap<T>(y0);
   // column starts of the XT lines: x and z of a cylinder index follow from
   // them (column x0 + j holds kz = 0..kc then -kc..-1)
   int csr[XT + 1];
@@ -946,10 +981,10 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
       out = s1[i];
     } else {                            // MODE 4: s0 to this slot and s1 to slot + 2
       out = s0[i];
-      dst[2 * ubf_var_elems<T>(g.nab_f, N) + ((size_t)((unsigned)a / TB) * N + y0) * TB + ((unsigned)a % TB)] =
+      dst[2 * ubf_var_elems<T>(g.nab_f, N) + ((size_t)((unsigned)a / TB) * N + y0) * TB + (((unsigned)a % TB) ^ swap)] =
           s1[i];
     }
-    dst[((size_t)((unsigned)a / TB) * N + y0) * TB + ((unsigned)a % TB)] = out;
+    dst[((size_t)((unsigned)a / TB) * N + y0) * TB + (((unsigned)a % TB) ^ swap)] = out;
   }
 }
 
@@ -1011,6 +1046,7 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
     const int c0 = act ? __ldg(g.colstart + x) : 0;
     const int kc = act ? (__ldg(g.colstart + x + 1) - c0 - 1) / 2 : -1;
     C* const dst0 = ub + box * g.bbox + (size_t)y * TB;
+    const int swap = ubf_swap<T>(y);
     const unsigned line = (l / PA::PW) * PA::BYTES + (l % PA::PW) * 16;   // the line's place in a buffer
 #pragma unroll 1
     for (int it = 0; it < ITEMS; it++) {
@@ -1038,11 +1074,11 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
       const int buf = it == 0 ? 0 : (it == 2 || it == 4) ? 3 - w : w;
       const unsigned o = buf * ZL::BUF + line;
       C v[E];
-      panel_load<T, N, R0>(smem, o, t, v);
+      panel_load<PA, R0>(smem, o, t, v);
       line_sync<P>();
-      panel_fft<T, N, false>(smem, o, t, tw, v);
+      panel_fft<PA, false>(smem, o, t, tw, v);
       if (it == 0) {
-        panel_store<T, N, RL>(smem, o, t, v);
+        panel_store<PA, RL>(smem, o, t, v);
         continue;
       }
       if (it < 3) {
@@ -1053,7 +1089,7 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
         for (int q = 0; q < E / RL; q++) {
           const int j = t + q * P;
           C p5[RL];
-          panel_read<T, N, false, RL, NSL>(smem, line ^ PA::template off<false>(j), line, j, p5);
+          panel_read<PA, false, RL, NSL>(smem, line ^ PA::template off<false>(j), line, j, p5);
 #pragma unroll
           for (int r = 0; r < RL; r++) {
             const T kz = T(j + r * NSL - (r < H ? 0 : N));
@@ -1073,17 +1109,19 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
           // z - N >= -kc at c0 + 2 kc + 1 + (z - N)
           const int z0 = h == 0 ? j : j - N / 2;
           const int a0 = h == 0 ? c0 + z0 : c0 + 2 * kc + 1 + z0;
+          if constexpr (NSL % TB == 0) {   // NS steps over whole runs of TB columns
+            C* const p0 = d + ((long)(a0 >> LT) * (N * TB) + ((a0 & (TB - 1)) ^ swap));
 #pragma unroll
-          for (int r = 0; r < H; r++) {
-            const bool in = h == 0 ? z0 + r * NSL <= kc : z0 + r * NSL >= -kc;
-            long e;
-            if constexpr (NSL % TB == 0) {   // NS steps over whole runs of TB columns
-              e = (long)(a0 >> LT) * (N * TB) + (a0 & (TB - 1)) + (long)r * ((long)(NSL / TB) * N * TB);
-            } else {
+            for (int r = 0; r < H; r++)
+              if (h == 0 ? z0 + r * NSL <= kc : z0 + r * NSL >= -kc)
+                p0[(long)r * ((long)(NSL / TB) * N * TB)] = v[q * RL + h * H + r];
+          } else {
+#pragma unroll
+            for (int r = 0; r < H; r++) {
               const int a = a0 + r * NSL;
-              e = (long)(a >> LT) * (N * TB) + (a & (TB - 1));
+              if (h == 0 ? z0 + r * NSL <= kc : z0 + r * NSL >= -kc)
+                d[(long)(a >> LT) * (N * TB) + ((a & (TB - 1)) ^ swap)] = v[q * RL + h * H + r];
             }
-            if (in) d[e] = v[q * RL + h * H + r];
           }
         }
       }
@@ -1164,7 +1202,7 @@ k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>*
 
 // ---------------------------------------------------------------------------
 // K5: y forward FFT + wavespace closure + proc4a (kstep 1) / proc4b (kstep 2)
-// grid (nab_f): one block = one ub block of TB_F columns
+// grid: one block = one slot of the forward ub layout, TB_F columns, or two
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void project3(C2<T>& u1, C2<T>& u2, C2<T>& u3, T kx, T ky, T kz,
@@ -1183,7 +1221,8 @@ __device__ __forceinline__ void project3(C2<T>& u1, C2<T>& u2, C2<T>& u3, T kx, 
 }
 
 template <typename T, int N, int KSTEP, int NC = 0, bool TCM = false>
-__global__ void __launch_bounds__(K5Launch<T, N, NC>::THREADS)
+__global__ void __launch_bounds__(TCM ? K5Launch<T, N, NC>::THREADS_TC : K5Launch<T, N, NC>::THREADS,
+                                  TCM ? 1 : K5Launch<T, N, NC>::MINB)
 k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __restrict__ u,
        C2<T>* __restrict__ un, const C2<T>* __restrict__ tw_g, double* __restrict__ efkz, TcArgs tca = TcArgs(),
        C2<T>* __restrict__ racc = nullptr) {
@@ -1196,7 +1235,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   //       forcing added to u
   //   14: racc += w*1/3, projected; un = u = racc, mean mode zeroed (the
   //       forcing that advanc_4.f adds to u is overwritten by that copy)
-  // grid (nab_f, boxes); forcing (efkz) is for single boxes only.
+  // grid (K5Launch::blocks(nab_f), boxes); forcing (efkz) is for single boxes only.
   // KSTEP = 0: transfer spectrum only (trfsp.f:62-83): the shell sums of
   // tfact Re(conj(un) . w) go to efkz[n/2] (shell ik = int(|k|/st.tdk + 1.5));
   // u and un are not written.
@@ -1209,36 +1248,82 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   // (wavespace_module.f:344-357) and advanced with the diffusivity factors
   // xdif ydif zdif (proc4a.f:508-522, proc4b.f:69-75), without projection
   using C = C2<T>;
-  constexpr int TB = Tiles<T>::TB_F;
+  using KL = K5Launch<T, N, NC>;
+  using PA = typename KL::PA;
+  constexpr bool PAD = TCM || !KL::SLOT;   // padded lines, else one-slot panels
+  constexpr int SC = Tiles<T>::TB_F, SPB = TCM ? 1 : KL::SPB, TB = SPB * SC, TBL = Tiles<T>::TBL_F, R = TBL / SC;
+  static_assert(R % SPB == 0, "a block's slots lie in one run");
   constexpr int NVF = 4 + NC;
-  constexpr int THREADS = K5Launch<T, N, NC>::THREADS;
+  constexpr int THREADS = TCM ? KL::THREADS_TC : KL::THREADS;
   constexpr int L = LS<T, N>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* buf = tw + FFTPlan<T, N>::TWSIZE;   // [4][TB] lines
-  double* thist = reinterpret_cast<double*>(buf + NVF * TB * L);   // KSTEP = 0: [n/2] shells
+  // one-slot panels, then the twiddles; or the twiddles, then padded lines
+  C* tw = reinterpret_cast<C*>(smem_raw + (PAD ? 0 : NVF * PA::BYTES));
+  C* buf = tw + FFTPlan<T, N>::TWSIZE;
+  // KSTEP = 0: [n/2] shells, behind both
+  double* thist = reinterpret_cast<double*>(buf + (PAD ? NVF * TB * L : 0));
   load_twiddles<T, N>(tw, tw_g);
   if constexpr (KSTEP == 0)
     for (int i = threadIdx.x; i < N / 2; i += THREADS) thist[i] = 0.0;
-  const int at = blockIdx.x, a0 = at * TB;
+  const int at = blockIdx.x * SPB, a0 = at * SC;
   for (int v = 0; v < NVF; v++) {
-    constexpr int TBL = Tiles<T>::TBL_F, R = TBL / TB;
-    const C* src = ub + (size_t)v * ubf_var_elems<T>(g.nab_f, N) + (size_t)(at / R) * N * TBL + (at % R) * TB;
-    for (int e = threadIdx.x; e < TB * N; e += THREADS) {
-      const int y = e / TB, l = e % TB;
-      cp_async_elem(buf + (v * TB + l) * L + padl<C, N>(y), src + y * TBL + l);
+    const C* src = ub + (size_t)v * ubf_var_elems<T>(g.nab_f, N) + (size_t)(at / R) * N * TBL + (at % R) * SC;
+    if constexpr (PAD) {
+      for (int e = threadIdx.x; e < TB * N; e += THREADS) {
+        const int y = e / TB, l = e % TB;
+        cp_async_elem(buf + (v * TB + l) * L + padl<C, N>(y), src + y * TBL + (l ^ ubf_swap<T>(y)));
+      }
+    } else {
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_raw + v * PA::BYTES);
+      for (int y = threadIdx.x; y < N; y += THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + y * 16), "l"(src + y * TBL) : "memory");
     }
   }
   const size_t vs = (size_t)g.xz_tot * N;
-  // the old state un of this thread's points
+  // the points of a thread, in PER steps of THREADS: column l, row y.  Where the
+  // threads divide a column, a step stays inside it
   constexpr int PER = (TB * N + THREADS - 1) / THREADS;
+  constexpr bool DIV = N % THREADS == 0;
+  auto col_of = [&](int q) { return DIV ? q / (N / THREADS > 0 ? N / THREADS : 1) : ((int)threadIdx.x + q * THREADS) / N; };
+  auto row_of = [&](int q) {
+    return DIV ? (int)threadIdx.x + q % (N / THREADS > 0 ? N / THREADS : 1) * THREADS : ((int)threadIdx.x + q * THREADS) % N;
+  };
+  // un is read after the transform (its registers are free then): bring the
+  // sphere's part of it into L2 meanwhile
+  if constexpr (!TCM) {
+    constexpr int LE = 128 / sizeof(C), LPC = N / LE;   // elements of a line, lines of a column
+    if constexpr (LPC > 0)
+      for (int i = threadIdx.x; i < (3 + NC) * TB * LPC; i += THREADS) {
+        const int y = i % LPC * LE, a = a0 + i / LPC % TB, v = i / LPC / TB;
+        if (a < g.xz_tot && (mask_ok(g, a, y, N) || mask_ok(g, a, y + LE - 1, N)))
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(un + v * vs + (size_t)a * N + y));
+      }
+  }
+  // constants of the block's columns, loaded here where a step's column is known
+  // when compiling, else point by point
+  struct ColK { int x, z, kym; C sxz; };
+  auto col_const = [&](int l) {
+    const int a = min(a0 + l, g.xz_tot - 1);
+    ColK c;
+    c.x = __ldg(g.ax + a);
+    c.z = __ldg(g.az + a);
+    c.kym = a0 + l < g.xz_tot ? __ldg(g.kymax + a) : -1;
+    c.sxz = cmul(__ldg(st.sz + c.z), __ldg(st.sx + c.x));
+    return c;
+  };
+  ColK ck[TB];
+  if constexpr (DIV) {
+#pragma unroll
+    for (int l = 0; l < TB; l++) ck[l] = col_const(l);
+  }
+  auto inside = [&](int y, int kym) { return y != N / 2 && (y > N / 2 ? N - y : y) <= kym; };
+  // the old state un of this thread's points
   C nb[PER][3 + NC];
   auto load_un = [&]() {
 #pragma unroll
     for (int q = 0; q < PER; q++) {
-      const int e = threadIdx.x + q * THREADS;
-      const int l = e / N, y = e % N, a = a0 + l;
-      if (e < TB * N && a < g.xz_tot && mask_ok(g, a, y, N)) {
+      const int l = col_of(q), y = row_of(q), a = a0 + l;
+      if (l < TB && (DIV ? inside(y, ck[DIV ? l : 0].kym) : a < g.xz_tot && mask_ok(g, a, y, N))) {
         const size_t o = (size_t)a * N + y;
 #pragma unroll
         for (int v = 0; v < 3 + NC; v++) nb[q][v] = un[v * vs + o];
@@ -1251,19 +1336,39 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   if constexpr (TCM) tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(buf + NVF * TB * L), tca);
   cp_async_wait_all();
   __syncthreads();
-  lines_fft<T, N, THREADS, TCM>(buf, NVF * TB, L, tw, w);
-  if constexpr (TCM) tc::teardown<NCOL>(w);
+  if constexpr (TCM) {
+    tc::fft1024_lines<THREADS>(buf, NVF * TB, L, w);
+    tc::teardown<NCOL>(w);
+  } else if constexpr (PAD) {
+    fft_lines<T, N, THREADS>(buf, NVF * TB, L, tw);
+  } else {
+    using PL = FFTPlan<T, N>;
+    constexpr int P = PL::P, R0 = PL::rad(0), RL = PL::rad(PL::NPASS - 1);
+    const int ln = threadIdx.x / P, t = threadIdx.x % P;
+    const unsigned o = (ln / TB) * PA::BYTES + (ln % TB) * PA::LX;
+    C v[PL::E];
+    panel_load<PA, R0>(smem_raw, o, t, v);
+    line_sync<P>();
+    panel_fft<PA, false>(smem_raw, o, t, tw, v);
+    panel_store<PA, RL>(smem_raw, o, t, v);
+    __syncthreads();
+  }
+  // transformed field v of column l at row y
+  auto val = [&](int v, int l, int y) -> C {
+    if constexpr (PAD) return buf[(v * TB + l) * L + padl<C, N>(y)];
+    else return *reinterpret_cast<const C*>(smem_raw + v * PA::BYTES + (PA::template off<false>(y) ^ (l * PA::LX)));
+  };
   // issued together after the transform (registers are free again), so each
   // thread waits once for all of its points
   load_un();
 #pragma unroll
   for (int q = 0; q < PER; q++) {
-    const int e = threadIdx.x + q * THREADS;
-    if (e >= TB * N) break;
-    const int l = e / N, y = e % N, a = a0 + l;
+    const int l = col_of(q), y = row_of(q), a = a0 + l;
+    if (l >= TB) break;
     if (a >= g.xz_tot) continue;
     const size_t o = (size_t)a * N + y;
-    if (!mask_ok(g, a, y, N)) {
+    const ColK cc = DIV ? ck[DIV ? l : 0] : col_const(l);
+    if (!inside(y, cc.kym)) {
       if constexpr (KSTEP != 0) {
         u[o] = cmk<C>(0, 0);
         u[vs + o] = cmk<C>(0, 0);
@@ -1272,14 +1377,12 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
       }
       continue;
     }
-    const int x = __ldg(g.ax + a), z = __ldg(g.az + a);
+    const int x = cc.x, z = cc.z;
     const int iky = kwave<N>(y), ikz = kwave<N>(z);
     const T kx = T(x), ky = T(iky), kz = T(ikz);
-    const int i = padl<C, N>(y);
-    const C V1 = buf[(0 * TB + l) * L + i], V2 = buf[(1 * TB + l) * L + i];
-    const C V3 = buf[(2 * TB + l) * L + i], V4 = buf[(3 * TB + l) * L + i];
+    const C V1 = val(0, l, y), V2 = val(1, l, y), V3 = val(2, l, y), V4 = val(3, l, y);
     // wavespace_vel.f:165-169
-    const C sxz = cmul(__ldg(st.sz + z), __ldg(st.sx + x));
+    const C sxz = cc.sxz;
     const C s = cconj(cmul(sxz, __ldg(st.sy + y)));
     const C sxyz = cmk<C>(-st.norm * s.x, -st.norm * s.y);
     const T tb = st.b22 * ky;
@@ -1382,7 +1485,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
       }
     }
     if constexpr (NC > 0) {
-      const C V5 = buf[(4 * TB + l) * L + i];
+      const C V5 = val(4, l, y);
       const C w4 = cmul(sxyz, V5);
       C n4 = nb[q][3], u4;
       if constexpr (KSTEP == 1) {

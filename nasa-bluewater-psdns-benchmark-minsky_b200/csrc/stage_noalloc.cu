@@ -185,8 +185,6 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   C* uz = (C*)(base + pl.uz);
   const C* twd = (const C*)(base + pl.tw);
   unsigned long long* vmx = (unsigned long long*)(base + pl.velmax);
-  constexpr int L = LS<T, N>::value;
-  constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
   {
     constexpr int TH = K1Launch<T, N>::THREADS;
     k_yinv<T, N><<<dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st>>>(geo, stb, u, ub, twd);
@@ -204,9 +202,9 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   {
     constexpr int TH = K5Launch<T, N, 0>::THREADS;
     if (kstep == 1)
-      k_yfwd<T, N, 1><<<geo.nab_f, TH, TWB + sizeof(C) * 4 * TL::TB_F * L, st>>>(geo, stb, ub, u, un, twd, nullptr);
+      k_yfwd<T, N, 1><<<K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st>>>(geo, stb, ub, u, un, twd, nullptr);
     else
-      k_yfwd<T, N, 2><<<geo.nab_f, TH, TWB + sizeof(C) * 4 * TL::TB_F * L, st>>>(geo, stb, ub, u, un, twd, nullptr);
+      k_yfwd<T, N, 2><<<K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st>>>(geo, stb, ub, u, un, twd, nullptr);
   }
   NA_CK(cudaGetLastError());
   unsigned long long vm_bits = 0;
