@@ -330,6 +330,7 @@ template <typename T, int N, int NC> struct Impl {
   using C = C2<T>;
   using TL = Tiles<T>;
   static constexpr int L = LS<T, N>::value;
+  static constexpr bool DEP = dep_launch(N, NC);
   static constexpr size_t TWB = sizeof(C) * FFTPlan<T, N>::TWSIZE;
   static size_t sm1() { return K1Launch<T, N>::SMEM; }
   using ZL = ZLaunch<T, N, 0>;
@@ -520,13 +521,12 @@ template <typename T, int N, int NC> struct Impl {
     {
       constexpr int TH = K1Launch<T, N>::THREADS;
       prof_mark(c, s, 0, 0);
-      k_yinv<T, N, false, NC><<<dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), TH, sm1(), c.stream>>>(g, st, u, ub, tw);
+      launch_dep<DEP>(k_yinv<T, N, false, NC>, dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), TH, sm1(), c.stream, g, st, u, ub, tw, TcArgs());
       prof_mark(c, s, 0, 1);
     }
     {
       prof_mark(c, s, 1, 0);
-      k_zinv<T, N, NC><<<k2_grid(3 + 3 * NC), ZL::THREADS, sm2(), c.stream>>>(
-          g, ub, uz, tw, st.b11, st.b33);
+      launch_dep<DEP>(k_zinv<T, N, NC>, k2_grid(3 + 3 * NC), ZL::THREADS, sm2(), c.stream, g, ub, uz, tw, st.b11, st.b33, TcArgs());
       prof_mark(c, s, 1, 1);
     }
     {
@@ -535,14 +535,13 @@ template <typename T, int N, int NC> struct Impl {
       // mean-gradient coefficients cb = beta * grad (init.f:42-45)
       const T cb1 = (T)(c.p.beta1 * c.p.grad[0]), cb2 = (T)(c.p.beta2 * c.p.grad[1]),
               cb3 = (T)(c.p.beta3 * c.p.grad[2]);
-      k_xchain<T, N, NC><<<dim3(N / K3Launch<T, N, NC>::TZ, N), TH, sm3(), c.stream>>>(g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax,
-                                                                    kstep == 1 ? 1 : 0, cb1, cb2, cb3);
+      launch_dep<DEP>(k_xchain<T, N, NC>, dim3(N / K3Launch<T, N, NC>::TZ, N), TH, sm3(), c.stream, g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1, cb2, cb3, TcArgs());
       prof_mark(c, s, 2, 1);
     }
     {
       prof_mark(c, s, 3, 0);
       const int tiles = k4_tiles(1);
-      k_zfwd<T, N, NC><<<k4_grid(tiles), ZL::THREADS, sm4(), c.stream>>>(g, uz, ub, tw, tiles, st.b11, st.b33);
+      launch_dep<DEP>(k_zfwd<T, N, NC>, k4_grid(tiles), ZL::THREADS, sm4(), c.stream, g, uz, ub, tw, tiles, st.b11, st.b33, TcArgs());
       prof_mark(c, s, 3, 1);
     }
     CK(cudaGetLastError());
@@ -614,10 +613,10 @@ template <typename T, int N, int NC> struct Impl {
       const C* tw = (const C*)c.d_tw;
       prof_mark(c, kstep - 1, 4, 0);
       switch (kstep) {
-        case 1: k_yfwd<T, N, 11><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 2: k_yfwd<T, N, 12><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 3: k_yfwd<T, N, 13><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        default: k_yfwd<T, N, 14><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r);
+        case 1: launch_dep<DEP>(k_yfwd<T, N, 11>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        case 2: launch_dep<DEP>(k_yfwd<T, N, 12>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        case 3: launch_dep<DEP>(k_yfwd<T, N, 13>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
+        default: launch_dep<DEP>(k_yfwd<T, N, 14>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r);
       }
       prof_mark(c, kstep - 1, 4, 1);
       CK(cudaGetLastError());
@@ -636,11 +635,9 @@ template <typename T, int N, int NC> struct Impl {
     constexpr int TH = K5Launch<T, N, NC>::THREADS;
     prof_mark(c, kstep - 1, 4, 0);
     if (kstep == 1)
-      k_yfwd<T, N, 1, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
-                                                        (const C*)c.d_tw, c.d_efkz);
+      launch_dep<DEP>(k_yfwd<T, N, 1, NC>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, TcArgs(), (C*)nullptr);
     else
-      k_yfwd<T, N, 2, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream>>>(g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un,
-                                                        (const C*)c.d_tw, c.d_efkz);
+      launch_dep<DEP>(k_yfwd<T, N, 2, NC>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, TcArgs(), (C*)nullptr);
     prof_mark(c, kstep - 1, 4, 1);
     CK(cudaGetLastError());
     return 0;

@@ -164,6 +164,38 @@ __device__ __forceinline__ void cp_async_elem(C* smem_dst, const C* gmem_src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// The kernels of a step follow one another on a stream, each on the results of
+// the one before.  launch_dep<true> lets a kernel's blocks start while the last
+// blocks of the kernel before still run, load what no kernel writes (the
+// twiddles), and wait in dep_wait until that kernel has completed and its
+// writes are visible; everything that a kernel of the step reads or writes
+// comes after dep_wait, which also lets the next kernel's blocks in once this
+// kernel's last ones have started.  (Launched otherwise, it does nothing.)
+// dep_launch: boxes of n <= 128 without a scalar, whose kernels are about as
+// short as the gaps between them (step of 64^3 FP32 118 -> 107 us, 128^3 235 ->
+// 221).  Where a kernel fills the GPU many times over, the blocks that wait
+// disturb it: 1024^3 64.0 -> 70.2 ms, 512^3 7.9 -> 8.5, 256^3 with a scalar and
+// particles 1.66 -> 1.71.
+__host__ __device__ constexpr bool dep_launch(int n, int nc) { return n <= 128 && nc == 0; }
+__device__ __forceinline__ void dep_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <bool DEP, typename... P, typename... A>
+inline void launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = DEP ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);   // the caller checks cudaGetLastError
+}
+
 // twiddles are copied asynchronously: every kernel calls cp_async_wait_all()
 // and __syncthreads() before its first FFT
 template <typename T, int N>
@@ -319,6 +351,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
   C* tw = reinterpret_cast<C*>(smem_raw);
   C* buf = tw + FFTPlan<T, N>::TWSIZE;
   load_twiddles<T, N>(tw, tw_g);
+  dep_wait();
   const int at = blockIdx.x, v = blockIdx.y;
   const int src = v < 3 ? v : 3;
   const int a0 = at * TB;
@@ -418,6 +451,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw + (TCM ? 0 : ZL::BUF));
   load_twiddles<T, N>(tw, tw_g);
+  dep_wait();
   // grid (n, lines / XT, fields * boxes)
   constexpr int NVZ = GRAD ? 2 : 3 + 3 * NC;
   const int y = blockIdx.x, x0 = blockIdx.y * XT, v = blockIdx.z % NVZ, box = blockIdx.z / NVZ;
@@ -845,6 +879,7 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
   C* bufE = bufW + NPAIR * L;
   C* bufF = bufE + NPAIR * L;
   load_twiddles<T, N>(tw, tw_g);
+  dep_wait();
   constexpr int NCOL = tc_cols(KL::LINES_TC);
   tc::Work w;
   if constexpr (TCM)
@@ -1035,6 +1070,7 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
   const int step = gridDim.x;
   int w = 1;   // buffer of P1 and P2; 3 - w: of P3 and P4
   load_twiddles<T, N>(tw, tw_g);
+  dep_wait();
   copy(0, 0, blockIdx.x);
   copy(w, 1, blockIdx.x);
   for (int tile = blockIdx.x; tile < ntiles; tile += step) {
@@ -1263,6 +1299,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   // KSTEP = 0: [n/2] shells, behind both
   double* thist = reinterpret_cast<double*>(buf + (PAD ? NVF * TB * L : 0));
   load_twiddles<T, N>(tw, tw_g);
+  dep_wait();
   if constexpr (KSTEP == 0)
     for (int i = threadIdx.x; i < N / 2; i += THREADS) thist[i] = 0.0;
   const int at = blockIdx.x * SPB, a0 = at * SC;

@@ -187,24 +187,22 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   unsigned long long* vmx = (unsigned long long*)(base + pl.velmax);
   {
     constexpr int TH = K1Launch<T, N>::THREADS;
-    k_yinv<T, N><<<dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st>>>(geo, stb, u, ub, twd);
+    launch_dep<dep_launch(N, 0)>(k_yinv<T, N>, dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st, geo, stb, u, ub, twd, TcArgs());
   }
   using ZL = ZLaunch<T, N, 0>;
-  k_zinv<T, N><<<dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st>>>(geo, ub, uz, twd);
+  launch_dep<dep_launch(N, 0)>(k_zinv<T, N>, dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st, geo, ub, uz, twd, T(1), T(1), TcArgs());
   {
     constexpr int TH = K3Launch<T, N, 0>::THREADS;
-    k_xchain<T, N><<<dim3(N / K3Launch<T, N, 0>::TZ, N), TH, K3Launch<T, N, 0>::SMEM, st>>>(
-        geo, uz, twd, stb.b11, stb.b22, stb.b33, vmx, kstep == 1 ? 1 : 0);
+    launch_dep<dep_launch(N, 0)>(k_xchain<T, N>, dim3(N / K3Launch<T, N, 0>::TZ, N), TH, K3Launch<T, N, 0>::SMEM, st, geo, uz, twd, stb.b11, stb.b22, stb.b33, vmx, kstep == 1 ? 1 : 0, T(0), T(0), T(0), TcArgs());
   }
   const int tiles = N * ZL::TILES;
-  k_zfwd<T, N><<<std::min(tiles, 148 * ZL::MINB4), ZL::THREADS, ZL::SMEM4, st>>>(geo, uz, ub, twd, tiles, stb.b11,
-                                                                                stb.b33);
+  launch_dep<dep_launch(N, 0)>(k_zfwd<T, N>, std::min(tiles, 148 * ZL::MINB4), ZL::THREADS, ZL::SMEM4, st, geo, uz, ub, twd, tiles, stb.b11, stb.b33, TcArgs());
   {
     constexpr int TH = K5Launch<T, N, 0>::THREADS;
     if (kstep == 1)
-      k_yfwd<T, N, 1><<<K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st>>>(geo, stb, ub, u, un, twd, nullptr);
+      launch_dep<dep_launch(N, 0)>(k_yfwd<T, N, 1>, K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st, geo, stb, ub, u, un, twd, (double*)nullptr, TcArgs(), (C*)nullptr);
     else
-      k_yfwd<T, N, 2><<<K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st>>>(geo, stb, ub, u, un, twd, nullptr);
+      launch_dep<dep_launch(N, 0)>(k_yfwd<T, N, 2>, K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st, geo, stb, ub, u, un, twd, (double*)nullptr, TcArgs(), (C*)nullptr);
   }
   NA_CK(cudaGetLastError());
   unsigned long long vm_bits = 0;
