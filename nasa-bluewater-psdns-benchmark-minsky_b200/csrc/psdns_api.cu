@@ -314,11 +314,16 @@ static void fill_shift_tables(Ctx& c) {
   }
 }
 
-static int upload_tables(Ctx& c) {
+// The staging buffer is reused by the next fill, so the copy is waited for,
+// unless the caller synchronises the stream before anything fills it again
+// (wait = false): within a step the velmax read lies between the shift tables
+// and the factors, and every entry point that steps ends with a
+// synchronisation.  The two waits of a step left the GPU idle while the host
+// returned to launch (64^3 FP64: HOSTFIG).
+static int upload_tables(Ctx& c, bool wait = true) {
   const size_t tot = c.prec == PSDNS_PREC_FP64 ? TabLayout<double>(c.n).total : TabLayout<float>(c.n).total;
   CK(cudaMemcpyAsync(c.d_tabs, c.h_tabs, tot, cudaMemcpyHostToDevice, c.stream));
-  // the staging buffer is reused by the next fill: wait for the copy
-  CK(cudaStreamSynchronize(c.stream));
+  if (wait) CK(cudaStreamSynchronize(c.stream));
   return 0;
 }
 
@@ -780,7 +785,7 @@ static int step_control(Ctx& c) {
 }
 
 // for(kfor,k2fo,k2fo,3) complex double -> device precision -> d_forc
-static int upload_forcing(Ctx& c, const double* tab) {
+static int upload_forcing(Ctx& c, const double* tab, bool wait = true) {
   const size_t nf = (size_t)c.kfor * c.k2fo * c.k2fo * 3;
   if (c.prec == PSDNS_PREC_FP64) {
     std::memcpy(c.h_forc, tab, nf * sizeof(double2));
@@ -789,7 +794,7 @@ static int upload_forcing(Ctx& c, const double* tab) {
     for (size_t i = 0; i < nf; i++) f[i] = make_float2((float)tab[2 * i], (float)tab[2 * i + 1]);
   }
   CK(cudaMemcpyAsync(c.d_forc, c.h_forc, nf * c.csz, cudaMemcpyHostToDevice, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+  if (wait) CK(cudaStreamSynchronize(c.stream));
   return 0;
 }
 
@@ -887,11 +892,11 @@ static int run_stage(Ctx& c, const Ops& o, int kstep, int* ctl_err) {
     }
     *ctl_err = step_control(c);
     if (c.prec == PSDNS_PREC_FP64) fill_factor_tables<double>(c); else fill_factor_tables<float>(c);
-    if (upload_tables(c)) return 1;
+    if (upload_tables(c, false)) return 1;
     if (c.p.kforce > 0) {
       // force.f, called after step at stage 1 (timestep_module.f:261-263)
       c.forcing.step(c.rng, c.dt, c.istart);
-      if (upload_forcing(c, c.forcing.table.data())) return 1;
+      if (upload_forcing(c, c.forcing.table.data(), false)) return 1;
       CK(cudaMemsetAsync(c.d_efkz, 0, sizeof(double) * 3 * (c.n / 2 + 2), c.stream));
     }
   }
@@ -2120,10 +2125,7 @@ int psdns_gpu_step(void* ctx, double* info) {
   c->jstep += 1;
   draw_shifts(*c);
   if (c->prec == PSDNS_PREC_FP64) fill_shift_tables<double>(*c); else fill_shift_tables<float>(*c);
-  if (c->jstep == 1) {
-    // factor tables are filled at stage 1; zero them before the first use
-  }
-  if (upload_tables(*c)) return 1;
+  if (upload_tables(*c, false)) return 1;
   int ctl = 0;
   for (int k = 1; k <= c->rk; k++)
     if (run_stage(*c, o, k, &ctl)) return 1;
@@ -2164,7 +2166,7 @@ int psdns_gpu_rk_stage(void* ctx, int32_t kstep, const double* gsh, const double
     CK(cudaMemsetAsync(c->d_velmax, 0, sizeof(unsigned long long), c->stream));
     if (c->p.kforce > 0) CK(cudaMemsetAsync(c->d_efkz, 0, sizeof(double) * 3 * (c->n / 2 + 2), c->stream));
   }
-  if (upload_tables(*c)) return 1;
+  if (upload_tables(*c, false)) return 1;
   if (c->p.kforce > 0) {
     // the driver passes this step's table (force.f); none means zero forcing
     std::vector<double> zero;
@@ -2331,7 +2333,7 @@ int psdns_gpu_particles_advance(void* ctx, const double* gsh1, double dt_prev) {
   for (int i = 0; i < 3; i++) c->gsh[i][0] = gsh1[i];
   c->dt = dt_prev;
   if (c->prec == PSDNS_PREC_FP64) fill_shift_tables<double>(*c); else fill_shift_tables<float>(*c);
-  if (upload_tables(*c)) return 1;
+  if (upload_tables(*c, false)) return 1;
   if (c->pin_nop > 0 && make_partin(*c)) return 1;
   if (c->np > 0 && o.particles(*c)) return 1;
   CK(cudaStreamSynchronize(c->stream));
