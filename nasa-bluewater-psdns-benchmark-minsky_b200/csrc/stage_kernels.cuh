@@ -1719,7 +1719,9 @@ __device__ __forceinline__ void spline_weights(double pos, double gfn, int n, in
                                       : fl / dn;
   const double jloc = fl - dn * floor(q);
   const double bfp = (jloc + px) - fl;
-  ib = (int)bfp;
+  // a position that is not finite (a run whose field has blown up) has no cell:
+  // cell 0, with weights that are not finite either
+  ib = bfp >= 0. && bfp <= dn ? (int)bfp : 0;
   const double t = bfp - ib;
   const double d6 = 1. / 6., tt = 2. / 3.;
   const double ym = 1. - t, yms = ym * ym;
