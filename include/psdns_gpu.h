@@ -353,7 +353,7 @@ int psdns_gpu_ensemble_step(void *ens, int32_t nsteps, double *info);
  * of FFTW's planner and wisdom, PSDNS/epfftw.f, PSDNS/wisdom.c): per class
  * of equal n, in the first steps of a fixed-dt class, the number of boxes
  * per launch, then the FFT tiles of the z transforms (x lines per block of
- * K2 and K4: the default, half, double; boxes of n <= 128), each candidate
+ * K2 and K4: the default, twice, four times; boxes of n <= 128), each candidate
  * timed over two real steps.  out[8 * cap] rows: n, boxes, tuned (0/1),
  * boxes per launch, K2 lines per block, K4 lines per block, step ms of the
  * all-default candidate, step ms of the choice; *nclasses = classes. */

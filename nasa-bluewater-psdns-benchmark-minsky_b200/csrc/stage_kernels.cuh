@@ -103,8 +103,8 @@ template <typename T> struct StageTables {
 };
 
 // per-precision tile sizes: TB_I = columns per K1 block (64 B runs in ub
-// for K2), TB_F = columns per K5 block, TZ = z lines per tile of the spline and
-// moment kernels.
+// for K2), TB_F = columns of a 16-byte slot of the forward ub layout (what K5
+// blocks are made of), TZ = z lines per tile of the spline and moment kernels.
 // Eight lines per K1 block keep two to three blocks resident per SM, so that
 // one block's copies overlap another's transforms; sixteen-line blocks (one
 // per SM) measured slower.
@@ -217,7 +217,7 @@ struct Launch {
   static_assert(THREADS % P == 0, "threads per line must divide the block");
 };
 
-// K1 and K4: one warp per line at n = 1024 FP32
+// K1: one warp per line at n = 1024 FP32
 template <typename T, int N>
 struct K1Launch : Launch<T, N, Tiles<T>::TB_I, 1024> {
   // its transposed store reads TB_I lines at two y a phase: a line stride of 2

@@ -34,7 +34,7 @@
 namespace psdns {
 namespace noalloc {
 
-// largest box the static scratch holds: 64^3 in FP64 (about 16.2 MB of scratch)
+// largest box the static scratch holds: 64^3 in FP64 (about 16.5 MB of scratch)
 constexpr int kMaxN = 64;
 constexpr size_t kBytes = PSDNS_NOALLOC_BYTES;
 
