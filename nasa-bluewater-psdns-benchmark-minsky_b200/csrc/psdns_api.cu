@@ -596,10 +596,10 @@ template <typename T, int N, int NC> struct Impl {
     constexpr int TH = K5Launch<T, N, NC>::THREADS_TC;
     prof_mark(c, kstep - 1, 4, 0);
     if (kstep == 1)
-      k_yfwd<T, N, 1, NC, true><<<c.nab_f, TH, sm5tc(), c.stream>>>(
+      k_yfwd<T, N, 1, NC, true><<<K5Launch<T, N, NC>::blocks_tc(c.nab_f), TH, sm5tc(), c.stream>>>(
           g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, ta);
     else
-      k_yfwd<T, N, 2, NC, true><<<c.nab_f, TH, sm5tc(), c.stream>>>(
+      k_yfwd<T, N, 2, NC, true><<<K5Launch<T, N, NC>::blocks_tc(c.nab_f), TH, sm5tc(), c.stream>>>(
           g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, ta);
     prof_mark(c, kstep - 1, 4, 1);
     CK(cudaGetLastError());

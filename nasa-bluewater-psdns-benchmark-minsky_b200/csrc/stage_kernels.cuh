@@ -283,9 +283,14 @@ struct K5Launch {
   // 0.204 ms against 0.157)
   static constexpr int WARPS = sizeof(T) == 4 || FFTPlan<T, N>::E <= 8 ? 24 : (SLOT ? 16 : 12);
   static constexpr int MINB = resident_blocks(SMEM, round_up(THREADS, 32), WARPS);
-  // tensor-core form: one slot in padded lines
-  static constexpr int LINES_TC = (4 + NC) * Tiles<T>::TB_F, THREADS_TC = Launch<T, N, LINES_TC, 1024>::THREADS;
-  static constexpr size_t SMEM_TC = TWB + sizeof(C2<T>) * LINES_TC * LS<T, N>::value + kTcTailBytes;
+  // tensor-core form: two slots in padded lines (sixteen lines, twenty with a
+  // scalar, for one set-up and one copy of the B operands).  The operand tiles
+  // overlay lines by fours and the tail follows, so the storage is whole tiles.
+  static constexpr int SPB_TC = 2;
+  static constexpr int blocks_tc(int nslots) { return (nslots + SPB_TC - 1) / SPB_TC; }
+  static constexpr int LINES_TC = (4 + NC) * SPB_TC * Tiles<T>::TB_F, STORE_TC = round_up(LINES_TC, 4);
+  static constexpr int THREADS_TC = Launch<T, N, LINES_TC, 1024>::THREADS;
+  static constexpr size_t SMEM_TC = TWB + sizeof(C2<T>) * STORE_TC * LS<T, N>::value + kTcTailBytes;
 };
 
 // Mixed-precision form of the stage kernels (template flag TCM, FP32 state
@@ -1287,7 +1292,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   using KL = K5Launch<T, N, NC>;
   using PA = typename KL::PA;
   constexpr bool PAD = TCM || !KL::SLOT;   // padded lines, else one-slot panels
-  constexpr int SC = Tiles<T>::TB_F, SPB = TCM ? 1 : KL::SPB, TB = SPB * SC, TBL = Tiles<T>::TBL_F, R = TBL / SC;
+  constexpr int SC = Tiles<T>::TB_F, SPB = TCM ? KL::SPB_TC : KL::SPB, TB = SPB * SC, TBL = Tiles<T>::TBL_F, R = TBL / SC;
   static_assert(R % SPB == 0, "a block's slots lie in one run");
   constexpr int NVF = 4 + NC;
   constexpr int THREADS = TCM ? KL::THREADS_TC : KL::THREADS;
@@ -1370,7 +1375,7 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __rest
   static_assert(!TCM || KSTEP != 0, "the transfer spectrum keeps the FP32 transform");
   constexpr int NCOL = tc_cols(NVF * TB);
   tc::Work w;
-  if constexpr (TCM) tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(buf + NVF * TB * L), tca);
+  if constexpr (TCM) tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(buf + KL::STORE_TC * L), tca);
   cp_async_wait_all();
   __syncthreads();
   if constexpr (TCM) {

@@ -57,3 +57,29 @@ def test_mixed_arm_against_fp64_at_1024(gpu_mod):
     assert errs["tc"][0] < 1e-4
     assert errs["tc"][1] < 1e-4
     assert errs["tc"][2] < 1e-4
+
+
+@pytest.mark.gpu
+def test_mixed_arm_with_a_scalar_at_1024(gpu_mod):
+    """Velocity and scalar of the tensor-core form against the plain FP32 step
+    (which tests/test_stage_layouts.py and tests/test_scalar.py compare with the
+    oracle).  The scalar starts from zero, so all of it has been through the
+    six transforms of a stage, at 4.5e-6 each: at most 3e-5."""
+    P = gpu_mod
+    ref = None
+    for dft in (P.DFT_FP32, P.DFT_TC_BF16X3):
+        p = params(P, 1024, P.PREC_FP32, dft)
+        p.nc, p.pr = 1, 0.7
+        p.grad[:] = (0.3, 1.0, -0.2)
+        s = P.Solver(p)
+        s.field_init(1234)
+        for _ in range(2):
+            assert s.step()["status"] == 0
+        got = s.get_state(P.FIELD_UN)
+        s.close()
+        if ref is None:
+            ref = got
+    for v in range(4):
+        err = math.sqrt(float(np.vdot(got[v] - ref[v], got[v] - ref[v]).real) / float(np.vdot(ref[v], ref[v]).real))
+        print(f"variable {v}: rel L2 {err:.2e}")
+        assert err < 3e-5, (v, err)

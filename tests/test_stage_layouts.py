@@ -4,6 +4,9 @@ form: the z-pencil panels (eight FP32 or four FP64 lines; n = 16 has one panel,
 of one slot (n >= 512) or two, the x chain's tiles of one pair or two and its
 batches with a scalar, the overlapped launches (n <= 128 without a scalar), and
 a CPU model of the panels' addresses."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -98,3 +101,14 @@ def test_positions_that_are_not_finite_stay_so(gpu_mod, prec):
     np.testing.assert_array_equal(out[1][0][ok], out[0][0][ok])
     np.testing.assert_array_equal(out[1][1][ok], out[0][1][ok])
     assert not np.isfinite(out[1][1][~ok]).all(axis=1).any()
+
+
+def test_layouts_of_the_kernels_header(gpu_mod, tmp_path):
+    """tests/stage_layouts.cu: the shared-memory storage of the tensor-core
+    forms covers their operand tiles."""
+    import build as pkg_build
+    exe = str(tmp_path / "stage_layouts")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "stage_layouts.cu")
+    subprocess.run([pkg_build.NVCC] + pkg_build.FLAGS + ["-O0", "-o", exe, src], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
