@@ -170,7 +170,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // twiddles), and wait in dep_wait until that kernel has completed and its
 // writes are visible; everything that a kernel of the step reads or writes
 // comes after dep_wait, which also lets the next kernel's blocks in once this
-// kernel's last ones have started.  (Launched otherwise, it does nothing.)
+// kernel's last ones have started.  (Launched otherwise, it does nothing.)  Since
+// the kernel before still writes while this one runs, u, un, ub and uz are read
+// with coherent loads (ld_step, plain loads, cp.async), not as read-only data
+// (__ldg, or a const __restrict__ kernel parameter), which is for the geometry and
+// the tables.
 // dep_launch: boxes of n <= 128 without a scalar, whose kernels are about as
 // short as the gaps between them (step of 64^3 FP32 118 -> 107 us, 128^3 235 ->
 // 221).  Where a kernel fills the GPU many times over, the blocks that wait
@@ -180,6 +184,23 @@ __host__ __device__ constexpr bool dep_launch(int n, int nc) { return n <= 128 &
 __device__ __forceinline__ void dep_wait() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+// A load of what the kernel before writes, for a kernel that may be launched
+// with launch_dep<DEP>.  Volatile like the waits, so that it stays behind
+// dep_wait.  Kernels that are never overlapped keep the read-only form: K2 of
+// 1024^3 FP32 4.03 ms, 4.39 with coherent loads (512^3 0.453 and 0.443; boxes of
+// n <= 128 the same with both).
+template <bool DEP> __device__ __forceinline__ float2 ld_step(const float2* p) {
+  if constexpr (!DEP) return __ldg(p);
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+template <bool DEP> __device__ __forceinline__ double2 ld_step(const double2* p) {
+  if constexpr (!DEP) return __ldg(p);
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
 }
 template <bool DEP, typename... P, typename... A>
 inline void launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
@@ -335,7 +356,7 @@ __device__ __forceinline__ void lines_fft(C2<T>* buf, int nlines, int ls, const 
 // ---------------------------------------------------------------------------
 template <typename T, int N, bool SPL = false, int NC = 0, bool TCM = false>
 __global__ void __launch_bounds__(K1Launch<T, N>::THREADS, TCM ? 2 : 3)
-k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restrict__ ub,
+k_yinv(Geo g, StageTables<T> st_all, const C2<T>* u, C2<T>* __restrict__ ub,
        const C2<T>* __restrict__ tw_g, TcArgs tca = TcArgs()) {
   // grid (nab_i, 3 + 2 nc, boxes)
   const int box = blockIdx.z;
@@ -385,7 +406,7 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ u, C2<T>* __restr
     C val = cmk<C>(0, 0);
     if (y != N / 2 && ky <= s.kym) {
       const C sh = cmul(__ldg(st.sy + y), s.sxz);
-      val = cmul(__ldg(s.col + y), sh);
+      val = cmul(ld_step<dep_launch(N, NC)>(s.col + y), sh);
     }
     return val;
   };
@@ -441,7 +462,7 @@ __host__ __device__ __forceinline__ int k1_blocks(int nab_i) { return nab_i; }
 template <typename T, int N, int NC = 0, bool GRAD = false, bool TCM = false, int PPBO = 0>
 __global__ void __launch_bounds__(TCM ? Launch<T, N, kTcXT2>::THREADS : ZLaunch<T, N, PPBO>::THREADS,
                                   TCM ? 2 : ZLaunch<T, N, PPBO>::MINB2)
-k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11 = T(1),
+k_zinv(Geo g, const C2<T>* ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11 = T(1),
        T b33 = T(1), TcArgs tca = TcArgs()) {
   // GRAD (two fields): uz slot 0 = i b11 kx u, slot 1 = i b33 kz w, the
   // gradients whose moments vgmomt.f takes (itransform.f:222-230)
@@ -478,7 +499,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
   auto fetch = [&](const Line& s, int z) {
     if (z > s.kc && z < N - s.kc) return cmk<C>(0, 0);
     const int a = s.ac + (z <= s.kc ? z : z - N + 2 * s.kc + 1);
-    return __ldg(src + ((size_t)((unsigned)a / TBL) * N + y) * TBL + ((unsigned)a % TBL));
+    return ld_step<dep_launch(N, NC)>(src + ((size_t)((unsigned)a / TBL) * N + y) * TBL + ((unsigned)a % TBL));
   };
   auto fix = [&](const Line& s, int z, C val) {
     if constexpr (GRAD) {
@@ -525,7 +546,7 @@ k_zinv(Geo g, const C2<T>* __restrict__ ub, C2<T>* __restrict__ uz, const C2<T>*
 #pragma unroll
           for (int r = 0; r < H; r++) {
             const bool in = h == 0 ? z0 + r * S0 <= s.kc : z0 + r * S0 >= -s.kc;
-            val[q * R0 + h * H + r] = in ? __ldg(p0 + (long)r * ((long)(S0 / TBL) * N * TBL)) : cmk<C>(0, 0);
+            val[q * R0 + h * H + r] = in ? ld_step<dep_launch(N, NC)>(p0 + (long)r * ((long)(S0 / TBL) * N * TBL)) : cmk<C>(0, 0);
           }
         }
     } else {
@@ -1041,7 +1062,7 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
 // One block barrier per field: it makes the field's copy visible, and frees
 // the buffer of the field before.
 template <typename T, int N, int NC, int PPBO>
-__device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub,
+__device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* uz, C2<T>* __restrict__ ub,
                                             unsigned char* smem, const C2<T>* __restrict__ tw_g, int ntiles, T b11,
                                             T b33) {
   using C = C2<T>;
@@ -1178,7 +1199,7 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* __restric
 template <typename T, int N, int NC = 0, bool TCM = false, int PPBO = 0>
 __global__ void __launch_bounds__(TCM ? Launch<T, N, 2 * kTcXT4, 1024>::THREADS : ZLaunch<T, N, PPBO>::THREADS,
                                   TCM ? 2 : ZLaunch<T, N, PPBO>::MINB4)
-k_zfwd(Geo g, const C2<T>* __restrict__ uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__ tw_g, int ntiles,
+k_zfwd(Geo g, const C2<T>* uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__ tw_g, int ntiles,
        T b11, T b33, TcArgs tca = TcArgs()) {
   // NC = 1: the scalar advection term (uz slot 5) goes to ub slot 4 without
   // derivatives (transform.f: i2f = 4+nc)
@@ -1264,7 +1285,7 @@ __device__ __forceinline__ void project3(C2<T>& u1, C2<T>& u2, C2<T>& u3, T kx, 
 template <typename T, int N, int KSTEP, int NC = 0, bool TCM = false>
 __global__ void __launch_bounds__(TCM ? K5Launch<T, N, NC>::THREADS_TC : K5Launch<T, N, NC>::THREADS,
                                   TCM ? 1 : K5Launch<T, N, NC>::MINB)
-k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* __restrict__ ub, C2<T>* __restrict__ u,
+k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* ub, C2<T>* __restrict__ u,
        C2<T>* __restrict__ un, const C2<T>* __restrict__ tw_g, double* __restrict__ efkz, TcArgs tca = TcArgs(),
        C2<T>* __restrict__ racc = nullptr) {
   // KSTEP = 11 .. 14: the RK4 sub-stages advanc_1 .. advanc_4

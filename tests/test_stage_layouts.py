@@ -5,6 +5,7 @@ of one slot (n >= 512) or two, the x chain's tiles of one pair or two and its
 batches with a scalar, the overlapped launches (n <= 128 without a scalar), and
 a CPU model of the panels' addresses."""
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -112,3 +113,27 @@ def test_layouts_of_the_kernels_header(gpu_mod, tmp_path):
     subprocess.run([pkg_build.NVCC] + pkg_build.FLAGS + ["-O0", "-o", exe, src], check=True)
     r = subprocess.run([exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_overlapped_kernels_read_the_steps_data_with_coherent_loads():
+    """A kernel launched with launch_dep runs beside the kernel before it, which
+    still writes what it reads after dep_wait.  Read-only loads (ld.global.nc:
+    __ldg, or a const __restrict__ parameter, for which the compiler may use them)
+    are defined only for data that nothing writes during the kernel: tables and
+    geometry, not u, un, ub, uz."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    path = os.path.join(root, "nasa-bluewater-psdns-benchmark-minsky_b200", "csrc", "stage_kernels.cuh")
+    with open(path) as f:
+        code = re.sub(r"//[^\n]*", "", f.read())
+    for arg in re.findall(r"__ldg\(\s*([^\s+,)\[]+)", code):
+        assert arg.startswith(("g.", "st.")) or arg == "p", arg   # p: ld_step of kernels never overlapped
+    assert len(re.findall(r"if constexpr \(!DEP\) return __ldg\(p\);", code)) == len(re.findall(r"__ldg\(p\)", code))
+    assert set(re.findall(r"\bld_step<([^;]*?)>\(", code)) == {"dep_launch(N, NC)"}
+    kernels = [(name, params) for name, params, body in re.findall(
+        r"__global__[^;{]*?\b(k_\w+)\(([^{]*?)\)\s*\{(.*?)\n\}", code, re.S) if re.search(r"dep_wait\(|zfwd_panels<", body)]
+    kernels += re.findall(r"\bvoid (zfwd_panels)\(([^{]*?)\)\s*\{", code)
+    assert {"k_yinv", "k_zinv", "k_xchain", "k_zfwd", "zfwd_panels", "k_yfwd"} == {name for name, _ in kernels}
+    for name, params in kernels:
+        for prm in params.split(","):
+            if re.search(r"\b(u|un|ub|uz|racc)\b\s*(=|$)", prm.strip()):
+                assert not ("const" in prm and "__restrict__" in prm), (name, prm.strip())
