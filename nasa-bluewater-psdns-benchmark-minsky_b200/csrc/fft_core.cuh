@@ -261,9 +261,23 @@ __device__ __forceinline__ void dft_tw(C* v, const C* __restrict__ tw) {
     a[i] = v[j];
   }
   {
+    // k = NS/2 turns by a quarter, whose tangent does not exist: its pair is
+    // marked by c = 2 and holds T = 1/2, and w = c (0 - i T).  The other tangents
+    // are at most N / 2 pi, and an operand that much below the type's largest
+    // value still passes.  (A tangent of 2^40 for the quarter would lose that much
+    // of the range; the selects cost 0.8% of a step at 1024^3 FP32, less at the
+    // other sizes.  Multiplying by 0 or 1 instead took the same in FP32, but 9%
+    // of K2 at 512^3 FP64.)
     const C w = tw[0];
+    const bool quarter = w.x > 1;
 #pragma unroll
-    for (int b = 0; b < R; b += 2) bfly<INV, false>(a[b], a[b + 1], w.x, w.y, a[b], a[b + 1]);
+    for (int b = 0; b < R; b += 2) {
+      const C o = a[b + 1], so = quarter ? cmk<C>(0, 0) : o;
+      const C u = INV ? cmk<C>(fma(-w.y, o.y, so.x), fma(w.y, o.x, so.y))
+                      : cmk<C>(fma(w.y, o.y, so.x), fma(-w.y, o.x, so.y));
+      a[b + 1] = cfma(-w.x, u, a[b]);
+      a[b] = cfma(w.x, u, a[b]);
+    }
   }
 #pragma unroll
   for (int l = 2; l <= LOG; l++) {
@@ -654,18 +668,13 @@ __device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t
 
 // Host: build the twiddle table of FFTPlan<T,N>: for every pass p >= 1 the
 // pairs (c, T) = (cos, tan) of the angle 2 pi (k + NS q') / (NS rho) of
-// dft_tw's combine steps, [row][k] with k < NS.  The angle pi/2 (rho = 2,
-// k = NS/2), whose tangent does not exist, is stored as c = 2^-40 (FP64
-// 2^-80), T = 1/c: c T = 1 exactly and the remaining c o.x is far below the
-// rounding of the sum it enters.
+// dft_tw's combine steps, [row][k] with k < NS; the angle pi/2 (rho = 2,
+// k = NS/2) as the pair (2, 1/2) that dft_tw knows it by.
 template <typename T, int N>
 void build_twiddles(C2<T>* out) {
   using PL = FFTPlan<T, N>;
   auto pair = [](long num, long den) {   // angle 2 pi num / den in [0, pi)
-    if (4 * num == den) {
-      const T c = std::ldexp(T(1), sizeof(T) == 8 ? -80 : -40);
-      return cmk<C2<T>>(c, T(1) / c);
-    }
+    if (4 * num == den) return cmk<C2<T>>(T(2), T(0.5));
     const long double ang = 2.0L * 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
     return cmk<C2<T>>((T)cosl(ang), (T)(sinl(ang) / cosl(ang)));
   };

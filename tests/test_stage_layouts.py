@@ -137,3 +137,28 @@ def test_overlapped_kernels_read_the_steps_data_with_coherent_loads():
         for prm in params.split(","):
             if re.search(r"\b(u|un|ub|uz|racc)\b\s*(=|$)", prm.strip()):
                 assert not ("const" in prm and "__restrict__" in prm), (name, prm.strip())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,nc", [(48, 0), (64, 1), (96, 0), (256, 1), (512, 0)])
+@pytest.mark.parametrize("prec,lg", [(0, 46), (1, 470)])
+def test_a_step_scales_with_powers_of_two(gpu_mod, n, nc, prec, lg):
+    """u -> s u, dt -> dt / s, nu -> s nu (with a scalar and its mean gradient times
+    s too) is a symmetry of the step, exact in floating point for a power of two
+    while nothing over- or underflows: the squares are below 2^(2 lg + 6), their
+    sums over the points of a plane below n^2 of that, and a twiddle pair
+    multiplies by at most tan = n / 2 pi on the way: 2^92 2^6 2^18 2^7 < 2^127."""
+    sc, out = 2.0 ** lg, []
+    for f in (1.0, sc):
+        s = gpu_mod.Solver(n=n, precision=prec, viscos=0.02 * f, cfl=-1.0, dt=0.125 / n / f, kshift=1, nc=nc, pr=0.7,
+                           grad=(0.3 * f, 0.0, f))
+        if not out:
+            s.field_init(77)
+            un = s.get_state()
+            if nc:
+                un[3] = 0.5 * un[1]
+        s.set_state(f * un)
+        assert s.step()["status"] == 0
+        out.append(s.get_state() / f)
+        s.close()
+    np.testing.assert_array_equal(out[0], out[1])
