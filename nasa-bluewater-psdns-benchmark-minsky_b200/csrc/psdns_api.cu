@@ -582,8 +582,9 @@ template <typename T, int N, int NC> struct Impl {
                                            cb2, cb3, ta);
     prof_mark(c, s, 2, 1);
     prof_mark(c, s, 3, 0);
-    k_zfwd<T, N, NC, true><<<dim3(N, (kxn + kTcXT4 - 1) / kTcXT4), Launch<T, N, 2 * kTcXT4, 1024>::THREADS, sm4tc(),
-                             c.stream>>>(g, uz, ub, tw, 0, st.b11, st.b33, ta);
+    k_zfwd<T, N, NC, true><<<dim3(N * (Panel<T, N>::PW / kTcXT4), ZL::NPAN),
+                             Launch<T, N, 2 * kTcXT4, 1024>::THREADS, sm4tc(), c.stream>>>(g, uz, ub, tw, 0, st.b11,
+                                                                                          st.b33, ta);
     prof_mark(c, s, 3, 1);
     CK(cudaGetLastError());
     return 0;

@@ -448,6 +448,22 @@ k_yinv(Geo g, StageTables<T> st_all, const C2<T>* u, C2<T>* __restrict__ ub,
 template <typename T>
 __host__ __device__ __forceinline__ int k1_blocks(int nab_i) { return nab_i; }
 
+// One bulk copy of what the block has written to shared memory (16-byte aligned,
+// a multiple of 16 bytes); called by every thread, last in a kernel.
+__device__ __forceinline__ void panel_to_global(void* dst, const void* src, unsigned bytes) {
+  // every thread's writes before the copy engine's reads
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst),
+                 "r"((unsigned)__cvta_generic_to_shared(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+    // the block's shared memory must outlive the copy's reads
+    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+  }
+}
+
 // ---------------------------------------------------------------------------
 // K2: cylinder unpack (zero fill) + z backward FFT, store to uz
 // grid (n, tiles of panels, fields)
@@ -516,17 +532,22 @@ k_zinv(Geo g, const C2<T>* ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__
   C* const plane = uz + ((size_t)v * N + y) * uz_slab<T>(N);
   if constexpr (TCM) {
     static_assert(kTcXT2 >= 4, "an operand tile overlays four lines");
+    static_assert(kTcXT2 == PA::PW, "a block's lines are one panel");
     constexpr int THREADS = Launch<T, N, XT>::THREADS, L = LS<T, N>::value;
     C* buf = tw + PL::TWSIZE;
-    const int nl = min(x0 + XT, g.kxn) - x0;
+    // the results go to global memory as a panel, like the FP32 form's, assembled
+    // over the operand tiles, which are free by then (9.0 ms at 1024^3; 9.8 with
+    // stores of 8 bytes a lane into the panel's rows)
+    unsigned char* const panel = reinterpret_cast<unsigned char*>(buf);
     tc::Work w;
     constexpr int NCOL = tc_cols(XT);
     tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(buf + XT * L), tca);
     tc::fft1024<THREADS>(
-        nl, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * L * sizeof(C)), begin,
-        [&](const Line& s, int z) { return fix(s, z, fetch(s, z)); }, [&](int l) { return x0 + l; },
-        [&](int x, int z, C val) { plane[uz_at<T, N>(x, z)] = cconj(val); });
+        XT, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * L * sizeof(C)), begin,
+        [&](const Line& s, int z) { return fix(s, z, fetch(s, z)); }, [&](int l) { return (unsigned)l * 16; },
+        [&](unsigned o, int z, C val) { *reinterpret_cast<C*>(panel + (PA::template off<false>(z) ^ o)) = cconj(val); });
     tc::teardown<NCOL>(w);
+    panel_to_global(plane + (size_t)blockIdx.y * PA::ELEMS, panel, PA::BYTES);
   } else {
     constexpr int R0 = PL::rad(0), E = PL::E, P = PL::P, RL = PL::rad(PL::NPASS - 1);
     const int l = threadIdx.x / P, t = threadIdx.x % P;
@@ -564,19 +585,8 @@ k_zinv(Geo g, const C2<T>* ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__
     const unsigned o = (l / PA::PW) * PA::BYTES + (l % PA::PW) * 16;
     panel_fft<PA, true>(smem_raw, o, t, tw, val);
     panel_store<PA, RL>(smem_raw, o, t, val);
-    // every thread's writes before the copy engine's reads
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int npan = min(ZL::PPB, ZL::NPAN - (int)blockIdx.y * ZL::PPB);
-      C* dst = plane + (size_t)blockIdx.y * ZL::PPB * PA::ELEMS;
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst),
-                   "r"((unsigned)__cvta_generic_to_shared(smem_raw)), "r"(npan * PA::BYTES)
-                   : "memory");
-      asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-      // the block's shared memory must outlive the copy's reads
-      asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-    }
+    const int npan = min(ZL::PPB, ZL::NPAN - (int)blockIdx.y * ZL::PPB);
+    panel_to_global(plane + (size_t)blockIdx.y * ZL::PPB * PA::ELEMS, smem_raw, npan * PA::BYTES);
   }
 }
 
@@ -990,15 +1000,24 @@ k_xchain(Geo g, C2<T>* __restrict__ uz, const C2<T>* __restrict__ tw_g, T b11, T
 // Output slots: 0 = d/dx(u^2-v^2)+d/dz(uw) partial,
 // 1 = uv, 2 = d/dx(uw)+d/dz(w^2-v^2), 3 = vw (y derivatives added in K5).
 // ---------------------------------------------------------------------------
-// tensor-core form: the nl lines from x0 of one field at row y to buf
-template <typename T, int N>
+// tensor-core form: the nl <= 4 lines from x0 (a multiple of 4) of one field at row
+// y to buf.  Consecutive threads take the entries of a slot, then the four slots
+// of a row, so a warp reads four 64-byte pieces (one line after the other it read
+// 16 bytes of sixteen rows: K4 of 1024^3 22.8 ms instead of 19.6)
+template <typename T, int N, int THREADS>
 __device__ __forceinline__ void zfwd_load(const C2<T>* __restrict__ uz, int slot, int y, int x0, int nl, C2<T>* buf,
                                           int L) {
-  const C2<T>* plane = uz + ((size_t)slot * N + y) * uz_slab<T>(N);
-  for (unsigned e = threadIdx.x; e < (unsigned)nl * N; e += blockDim.x) {
-    const unsigned z = e % N, l = e / N;
-    cp_async_elem(buf + l * L + padl<C2<T>, N>(z), plane + uz_at<T, N>(x0 + l, z));
-  }
+  using PA = Panel<T, N>;
+  static_assert(PA::PW % kTcXT4 == 0 && kTcXT4 == 4, "four lines are one aligned half of a row's slots");
+  constexpr int Z = THREADS / 4;   // entries of a line from one step of a thread to the next
+  static_assert(THREADS % 4 == 0 && N % Z == 0 && Z % 32 == 0 && Z / PA::ZS % 8 == 0, "a step keeps the line");
+  const unsigned rho = threadIdx.x / (4 * PA::ZS), l = (threadIdx.x / PA::ZS ^ PA::sw(rho)) & 3;
+  if (l >= (unsigned)nl) return;
+  const unsigned z = rho * PA::ZS + threadIdx.x % PA::ZS;
+  const C2<T>* src = uz + ((size_t)slot * N + y) * uz_slab<T>(N) + uz_at<T, N>(x0 + l, z);
+  C2<T>* dst = buf + l * L + padl<C2<T>, N>(z);
+#pragma unroll
+  for (int i = 0; i < N / Z; i++) cp_async_elem(dst + i * padl<C2<T>, N>(Z), src + i * (Z / PA::ZS * PA::ROW));
 }
 
 template <typename T, int N, int MODE, int XT>
@@ -1195,7 +1214,7 @@ __device__ __forceinline__ void zfwd_panels(const Geo& g, const C2<T>* uz, C2<T>
 
 // PPBO > 0: panels per block (ensemble tuner).  grid: the tiles (n y rows x
 // TILES x boxes), or as many blocks as stay resident; tensor-core form:
-// (n, lines / kTcXT4)
+// (n times the halves of a panel, panels)
 template <typename T, int N, int NC = 0, bool TCM = false, int PPBO = 0>
 __global__ void __launch_bounds__(TCM ? Launch<T, N, 2 * kTcXT4, 1024>::THREADS : ZLaunch<T, N, PPBO>::THREADS,
                                   TCM ? 2 : ZLaunch<T, N, PPBO>::MINB4)
@@ -1209,13 +1228,18 @@ k_zfwd(Geo g, const C2<T>* uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__
     zfwd_panels<T, N, NC, PPBO>(g, uz, ub, smem_raw, tw_g, ntiles, b11, b33);
   } else {
     // tensor-core form: rounds of two fields through shared memory
+    using PA = Panel<T, N>;
     constexpr int XT = kTcXT4, THREADS = Launch<T, N, 2 * XT, 1024>::THREADS, L = LS<T, N>::value;
     static_assert(XT >= 4, "an operand tile overlays four lines of s0 or s1");
     C* tw = reinterpret_cast<C*>(smem_raw);
     C* s0 = tw + FFTPlan<T, N>::TWSIZE;
     C* s1 = s0 + XT * L;
     load_twiddles<T, N>(tw, tw_g);
-    const int y = blockIdx.x, x0 = blockIdx.y * XT, x1 = min(x0 + XT, g.kxn), nl = x1 - x0;
+    // the blocks of a panel's two halves are neighbours, so that what one reads of
+    // a 128-byte row meets the other's part in L2
+    constexpr int H = PA::PW / XT;
+    const int y = blockIdx.x / H, x0 = (blockIdx.y * H + blockIdx.x % H) * XT, x1 = min(x0 + XT, g.kxn), nl = x1 - x0;
+    if (nl <= 0) return;   // a half beyond kxn
     constexpr int NCOL = tc_cols(2 * XT);
     tc::Work w;
     tc_begin<NCOL>(w, reinterpret_cast<unsigned char*>(s1 + XT * L), tca);
@@ -1228,23 +1252,23 @@ k_zfwd(Geo g, const C2<T>* uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__
       }
     };
     // round 1: P5 -> s0, P1 -> s1
-    zfwd_load<T, N>(uz, 4, y, x0, nl, s0, L);
-    zfwd_load<T, N>(uz, 0, y, x0, nl, s1, L);
+    zfwd_load<T, N, THREADS>(uz, 4, y, x0, nl, s0, L);
+    zfwd_load<T, N, THREADS>(uz, 0, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
     both();
     zfwd_store<T, N, 0, XT>(g, s0, s1, L, ub, 0, y, x0, x1, b11, b33);
     __syncthreads();
     // round 2: P3 -> s1
-    zfwd_load<T, N>(uz, 2, y, x0, nl, s1, L);
+    zfwd_load<T, N, THREADS>(uz, 2, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
     lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
     zfwd_store<T, N, 1, XT>(g, s0, s1, L, ub, 2, y, x0, x1, b11, b33);
     __syncthreads();
     // round 3: P2 -> s0, P4 -> s1
-    zfwd_load<T, N>(uz, 1, y, x0, nl, s0, L);
-    zfwd_load<T, N>(uz, 3, y, x0, nl, s1, L);
+    zfwd_load<T, N, THREADS>(uz, 1, y, x0, nl, s0, L);
+    zfwd_load<T, N, THREADS>(uz, 3, y, x0, nl, s1, L);
     cp_async_wait_all();
     __syncthreads();
     both();
@@ -1252,7 +1276,7 @@ k_zfwd(Geo g, const C2<T>* uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__
     zfwd_store<T, N, 4, XT>(g, s0, s1, L, ub, 1, y, x0, x1, b11, b33);
     if constexpr (NC > 0) {
       __syncthreads();
-      zfwd_load<T, N>(uz, 5, y, x0, nl, s1, L);
+      zfwd_load<T, N, THREADS>(uz, 5, y, x0, nl, s1, L);
       cp_async_wait_all();
       __syncthreads();
       lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
