@@ -573,15 +573,20 @@ template <typename T_, int N_, bool SLOT1 = false> struct Panel {
     const unsigned rho = i / ZS;
     return rho * (ROW * sizeof(C)) + sw(rho) * LX + (i % ZS) * sizeof(C);
   }
-  // element a + B of the line at byte offset o (panel offset + LX x); the bits
-  // of a and B are disjoint for N = 2^k
-  template <bool XCH, unsigned B> __device__ __forceinline__ static C& at(unsigned char* smem, unsigned oa, unsigned o, unsigned a) {
+  // byte offset of element a + B of the line at byte offset o (panel offset + LX
+  // x), oa = o ^ off(a); the bits of a and B are disjoint for N = 2^k
+  template <bool XCH, unsigned B>
+  __host__ __device__ __forceinline__ static constexpr unsigned addr(unsigned oa, unsigned o, unsigned a) {
     if constexpr (POW2) {
       constexpr unsigned c = off<XCH>(B);
-      return *reinterpret_cast<C*>(smem + (oa ^ (c & LOW)) + (c & ~LOW));
+      return (oa ^ (c & LOW)) + (c & ~LOW);
     } else {
-      return *reinterpret_cast<C*>(smem + (o & ~127u) + (off<XCH>(a + B) ^ (o & 127)));
+      return (o & ~127u) + (off<XCH>(a + B) ^ (o & 127));
     }
+  }
+  template <bool XCH, unsigned B>
+  __device__ __forceinline__ static C& at(unsigned char* smem, unsigned oa, unsigned o, unsigned a) {
+    return *reinterpret_cast<C*>(smem + addr<XCH, B>(oa, o, a));
   }
 };
 

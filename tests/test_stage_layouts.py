@@ -16,11 +16,11 @@ def _eps(prec):
     return 2.0 ** -52 if prec else 2.0 ** -23
 
 
-def _run(gpu_mod, oracle_mod, n, nc, precs, nu=0.02):
+def _run(gpu_mod, oracle_mod, n, nc, precs, nu=0.02, rkmethod=2):
     # velmax is about 6 n for this field: a Courant number velmax dt / 2 pi of
     # about 1/4 (step.f refuses numbers above 1)
     dt = 0.25 / n
-    o = oracle_mod.Oracle(n, nu, cfl=-1.0, dt=dt, kshift=1)
+    o = oracle_mod.Oracle(n, nu, cfl=-1.0, dt=dt, kshift=1, rkmethod=rkmethod)
     if nc:
         o.set_scalar(pr=0.7, grad=(0.3, 0.0, 1.0))
     un = o.field_init(77)
@@ -32,14 +32,14 @@ def _run(gpu_mod, oracle_mod, n, nc, precs, nu=0.02):
     o.close()
     for prec in precs:
         s = gpu_mod.Solver(n=n, precision=prec, viscos=nu, cfl=-1.0, dt=dt, kshift=1, nc=nc, pr=0.7,
-                           grad=(0.3, 0.0, 1.0))
+                           grad=(0.3, 0.0, 1.0), rkmethod=rkmethod)
         s.set_state(un)
         assert s.step()["status"] == 0
         got = s.get_state()
         s.close()
         # a transform of n^3 points adds at most about log2(n^3) roundings to a
-        # mode, a stage has one there and one back, a step two stages
-        bound = 4 * np.log2(float(n) ** 3) * _eps(prec)
+        # mode, a stage has one there and one back, a step two stages (RK4 four)
+        bound = 2 * rkmethod * np.log2(float(n) ** 3) * _eps(prec)
         for v in range(3 + nc):
             err = np.linalg.norm(got[v] - want[v]) / np.linalg.norm(want[v])
             assert err < bound, (n, nc, prec, v, err, bound)
@@ -55,6 +55,18 @@ def test_step_against_oracle(gpu_mod, oracle_mod, n, nc):
 @pytest.mark.gpu
 def test_step_of_512_against_oracle(gpu_mod, oracle_mod):
     _run(gpu_mod, oracle_mod, 512, 0, (0, 1))
+
+
+@pytest.mark.gpu
+def test_step_of_512_with_a_scalar_against_oracle(gpu_mod, oracle_mod):
+    """One slot of five fields: 160 threads in FP32, which do not divide a column."""
+    _run(gpu_mod, oracle_mod, 512, 1, (0, 1))
+
+
+@pytest.mark.gpu
+def test_rk4_step_of_512_against_oracle(gpu_mod, oracle_mod):
+    """advanc_1..4 as epilogues of the one-slot y transforms; four stages."""
+    _run(gpu_mod, oracle_mod, 512, 0, (0, 1), rkmethod=4)
 
 
 @pytest.mark.parametrize("zs,pw", [(2, 8), (1, 4)])
@@ -105,8 +117,10 @@ def test_positions_that_are_not_finite_stay_so(gpu_mod, prec):
 
 
 def test_layouts_of_the_kernels_header(gpu_mod, tmp_path):
-    """tests/stage_layouts.cu: the shared-memory storage of the tensor-core
-    forms covers their operand tiles."""
+    """tests/stage_layouts.cu, built against the kernels' header: every element of
+    a panel has its own place in both orders (z panels and one-slot panels), the
+    split addresses of every access of every pass are those places, and the
+    shared-memory storage of the tensor-core forms covers their operand tiles."""
     import build as pkg_build
     exe = str(tmp_path / "stage_layouts")
     src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "stage_layouts.cu")
