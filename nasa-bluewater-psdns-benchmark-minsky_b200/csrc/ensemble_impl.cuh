@@ -111,7 +111,8 @@ template <typename T, int N> struct EnsImpl {
   static void k2(EnsClass& e, const Geo& g, const C* ub, C* uz, const C* tw, const StageTables<T>& st, int nb) {
     if constexpr (F == 1 || kTiles) {
       using Z = ZLaunch<T, N, ppb<F>()>;
-      launch_dep<I::DEP>(k_zinv<T, N, 0, false, false, ppb<F>()>, dim3(N, Z::TILES, 3 * nb), Z::THREADS, Z::SMEM2, e.stream, g, ub, uz, tw, st.b11, st.b33, TcArgs());
+      launch_dep<I::DEP>(k_zinv<T, N, 0, false, false, ppb<F>()>, dim3(N, Z::TILES, 3 * nb), Z::THREADS, Z::SMEM2,
+                         e.stream, g, ub, uz, tw, st.b11, st.b33, TcArgs());
     }
   }
   template <int F>
@@ -119,7 +120,8 @@ template <typename T, int N> struct EnsImpl {
     if constexpr (F == 1 || kTiles) {
       using Z = ZLaunch<T, N, ppb<F>()>;
       const int tiles = N * Z::TILES * nb;
-      launch_dep<I::DEP>(k_zfwd<T, N, 0, false, ppb<F>()>, std::min(tiles, 148 * Z::MINB4), Z::THREADS, Z::SMEM4, e.stream, g, uz, ub, tw, tiles, st.b11, st.b33, TcArgs());
+      launch_dep<I::DEP>(k_zfwd<T, N, 0, false, ppb<F>()>, std::min(tiles, 148 * Z::MINB4), Z::THREADS, Z::SMEM4,
+                         e.stream, g, uz, ub, tw, tiles, st.b11, st.b33, TcArgs());
     }
   }
 
@@ -131,13 +133,16 @@ template <typename T, int N> struct EnsImpl {
     C* u = (C*)e.d_u + (size_t)b0 * e.st_elems;
     C* ub = (C*)e.d_ub + (size_t)b0 * e.ub_elems;
     C* uz = (C*)e.d_uz + (size_t)b0 * e.uz_elems;
-    launch_dep<I::DEP>(k_yinv<T, N>, dim3(k1_blocks<T>(e.nab_i), 3, nb), K1Launch<T, N>::THREADS, I::sm1(), e.stream, g, st, u, ub, tw, TcArgs());
+    launch_dep<I::DEP>(k_yinv<T, N>, dim3(k1_blocks<T>(e.nab_i), 3, nb), K1Launch<T, N>::THREADS, I::sm1(), e.stream,
+                       g, st, u, ub, tw, TcArgs());
     switch (kTiles ? e.k2v : 0) {
       case 1: k2<2>(e, g, ub, uz, tw, st, nb); break;
       case 2: k2<4>(e, g, ub, uz, tw, st, nb); break;
       default: k2<1>(e, g, ub, uz, tw, st, nb);
     }
-    launch_dep<I::DEP>(k_xchain<T, N>, dim3(N / K3Launch<T, N, 0>::TZ, N, nb), K3Launch<T, N, 0>::THREADS, I::sm3(), e.stream, g, uz, tw, st.b11, st.b22, st.b33, e.d_velmax + b0, kstep == 1 ? 1 : 0, T(0), T(0), T(0), TcArgs());
+    launch_dep<I::DEP>(k_xchain<T, N>, dim3(N / K3Launch<T, N, 0>::TZ, N, nb), K3Launch<T, N, 0>::THREADS, I::sm3(),
+                       e.stream, g, uz, tw, st.b11, st.b22, st.b33, e.d_velmax + b0, kstep == 1 ? 1 : 0, T(0), T(0),
+                       T(0), TcArgs());
     switch (kTiles ? e.k4v : 0) {
       case 1: k4<2>(e, g, uz, ub, tw, st, nb); break;
       case 2: k4<4>(e, g, uz, ub, tw, st, nb); break;
@@ -154,10 +159,9 @@ template <typename T, int N> struct EnsImpl {
     const C* ub = (const C*)e.d_ub + (size_t)b0 * e.ub_elems;
     C* u = (C*)e.d_u + (size_t)b0 * e.st_elems;
     C* un = (C*)e.d_un + (size_t)b0 * e.st_elems;
-    if (kstep == 1)
-      launch_dep<I::DEP>(k_yfwd<T, N, 1>, dim3(K5Launch<T, N, 0>::blocks(e.nab_f), nb), TH, I::sm5(), e.stream, g, st, ub, u, un, (const C*)e.d_tw, (double*)nullptr, TcArgs(), (C*)nullptr);
-    else
-      launch_dep<I::DEP>(k_yfwd<T, N, 2>, dim3(K5Launch<T, N, 0>::blocks(e.nab_f), nb), TH, I::sm5(), e.stream, g, st, ub, u, un, (const C*)e.d_tw, (double*)nullptr, TcArgs(), (C*)nullptr);
+    const dim3 grid(K5Launch<T, N, 0>::blocks(e.nab_f), nb);
+    launch_dep<I::DEP>(kstep == 1 ? k_yfwd<T, N, 1> : k_yfwd<T, N, 2>, grid, TH, I::sm5(), e.stream, g, st, ub, u, un,
+                       (const C*)e.d_tw, (double*)nullptr, TcArgs(), (C*)nullptr);
     CK(cudaGetLastError());
     return 0;
   }

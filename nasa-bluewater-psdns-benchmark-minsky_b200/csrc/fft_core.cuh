@@ -3,26 +3,32 @@
 // Replaces the FFTW 1-D transforms the reference plans in PSDNS/epfftw.f
 // (plan4_p1/plan4_p3 along y, plan2_kx/plan2_xk along z, plan3_p2c/plan1_p2b
 // along x).  Unnormalised forward transform X_k = sum_j x_j exp(-2 pi i jk/N);
-// the backward transform is obtained by conjugating input and output.
+// INV: the backward one, with conjugate twiddles in the same passes (K1 and K2;
+// the x chain, whose pairs of real lines come conjugated, transforms forward both
+// ways).
 //
 // Algorithm: Stockham auto-sort with mixed register radices.  A line of N
 // points is split into passes of radix R_p (product = N).  In every pass each
 // thread owns E/R_p butterflies of radix R_p whose operands it holds in
 // registers; the radix-R kernels are unrolled at compile time.  Between passes
-// data goes through shared memory in place: all operands are read, the block
-// synchronises, then all results are written.  Element i of a line lives at
+// data goes through shared memory in place: all operands are read, the threads of
+// the line synchronise, then all results are written.  Element i of a line lives at
 // padl(i), which keeps the strided writes of the first pass from serialising
 // on one bank.
 //
 // What bounds the transforms inside the kernels is the number of instructions
-// issued, not the FMA pipe (the x chain issued 0.59 per cycle and scheduler at
-// 40% of that pipe), so the arithmetic is arranged for few instructions:
+// issued, not the FMA pipe (with scalar arithmetic and the twiddles multiplied
+// onto the operands the x chain issued 0.59 per cycle and scheduler at 40% of that
+// pipe; in this form 0.60, in a quarter fewer instructions: 914 -> 672 million a
+// launch at 512^3 FP32), so the arithmetic is arranged for few instructions:
 //  * Complex sums, and the sums of a twiddled butterfly, are packed FP32 pair
 //    instructions (add, subtract, fma of (re, im)): one issue slot instead of
 //    two, with the rounding of the scalar forms.
 //  * A butterfly e +- w o with w = c (1 - i T), T = tan, is u = o (1 - i T)
 //    (two scalar fma) and e +- c u (two packed fma): 4 instructions instead of
-//    8.  Each component is rounded twice instead of three times.
+//    8.  Each component is rounded twice instead of three times.  (The form of
+//    Linzer and Feig, Math. Comp. 60, 1993, and Goedecker, SIAM J. Sci. Comput.
+//    18, 1997, for fused multiply-add machines.)
 //  * The inter-pass twiddles are not applied to the operands before a radix-R
 //    kernel but inside its butterflies, stage by stage, where a twiddle costs
 //    nothing beyond the table load: a radix-R pass needs R/2 pairs (c, T) per
@@ -314,9 +320,6 @@ __host__ __device__ constexpr int plan_rad(int N, bool dbl, int p) {
     const int a = (K + 2) / 3, b = (K - a + 1) / 2, c = K - a - b;
     return p == 0 ? (1 << a) : (p == 1 ? (1 << b) : (p == 2 ? (1 << c) : 1));
   }
-  if (N == 6) return p == 0 ? 6 : 1;
-  if (N == 12) return p == 0 ? 3 : (p == 1 ? 4 : 1);
-  if (N == 24) return p == 0 ? 6 : (p == 1 ? 4 : 1);
   if (N == 48) return p == 0 ? 12 : (p == 1 ? 4 : 1);
   if (N == 96) return p == 0 ? 12 : (p == 1 ? 8 : 1);
   return 1;
@@ -342,8 +345,7 @@ __host__ __device__ constexpr int plan_twoff(int N, bool dbl, int p) {
 
 template <typename T, int N> struct FFTPlan {
   static constexpr bool DBL = sizeof(T) == 8;
-  static_assert(is_pow2(N) || N == 48 || N == 96 || N == 24 || N == 12 || N == 6,
-                "N must be a power of two (or 6*2^k up to 96)");
+  static_assert(is_pow2(N) || N == 48 || N == 96, "N must be a power of two, 48 or 96");
   static constexpr int NPASS = plan_npass(N, DBL);
   static constexpr int rad(int p) { return plan_rad(N, DBL, p); }
   static constexpr int E = plan_e(N, DBL);
@@ -591,14 +593,16 @@ template <typename T_, int N_, bool SLOT1 = false> struct Panel {
 };
 
 template <typename PA, bool XCH, int R, int STEP, int r = 0>
-__device__ __forceinline__ void panel_read(unsigned char* smem, unsigned oa, unsigned o, unsigned a, typename PA::C* v) {
+__device__ __forceinline__ void panel_read(unsigned char* smem, unsigned oa, unsigned o, unsigned a,
+                                           typename PA::C* v) {
   if constexpr (r < R) {
     v[r] = PA::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a);
     panel_read<PA, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
   }
 }
 template <typename PA, bool XCH, int R, int STEP, int r = 0>
-__device__ __forceinline__ void panel_write(unsigned char* smem, unsigned oa, unsigned o, unsigned a, const typename PA::C* v) {
+__device__ __forceinline__ void panel_write(unsigned char* smem, unsigned oa, unsigned o, unsigned a,
+                                            const typename PA::C* v) {
   if constexpr (r < R) {
     PA::template at<XCH, (unsigned)r * STEP>(smem, oa, o, a) = v[r];
     panel_write<PA, XCH, R, STEP, r + 1>(smem, oa, o, a, v);
@@ -631,7 +635,8 @@ __device__ __forceinline__ void panel_store(unsigned char* smem, unsigned o, int
 // v[q R + r]) out; afterwards every slot of the line has been read.  Called by
 // whole warps.
 template <typename PA, bool INV>
-__device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t, const typename PA::C* tw, typename PA::C* v) {
+__device__ __forceinline__ void panel_fft(unsigned char* smem, unsigned o, int t, const typename PA::C* tw,
+                                          typename PA::C* v) {
   using PL = typename PA::PL;
   static_assert(PL::NPASS >= 2, "load and store passes must differ");
   constexpr int N = PA::N, E = PL::E, P = PL::P, R0 = PL::rad(0);

@@ -408,12 +408,10 @@ template <typename T, int N, int NC> struct Impl {
     const C* tw = (const C*)c.d_tw;
     C* ub = (C*)c.d_ub;
     C* uz = (C*)c.d_uz;
-    const int kxn = c.g.kxn;
     prof_mark(c, 0, 5, 0);
-    k_yinv<T, N, true><<<dim3(k1_blocks<T>(c.nab_i), 3), K1Launch<T, N>::THREADS, sm1(), c.stream>>>(g, st, (const C*)c.d_u,
-                                                                                               ub, tw);
-    k_zinv<T, N><<<k2_grid(3), ZL::THREADS, sm2(), c.stream>>>(
-        g, ub, uz, tw);
+    k_yinv<T, N, true><<<dim3(k1_blocks<T>(c.nab_i), 3), K1Launch<T, N>::THREADS, sm1(), c.stream>>>(
+        g, st, (const C*)c.d_u, ub, tw);
+    k_zinv<T, N><<<k2_grid(3), ZL::THREADS, sm2(), c.stream>>>(g, ub, uz, tw);
     using V4 = typename V4T<T>::type;
     k_xspline<T, N><<<dim3(c.nzt, N), Launch<T, N, 2 * TL::TZ>::THREADS, smxs(), c.stream>>>(g, uz, (V4*)c.d_bs, tw);
     const double pi = 4. * std::atan(1.);
@@ -444,11 +442,9 @@ template <typename T, int N, int NC> struct Impl {
     const C* tw = (const C*)c.d_tw;
     C* ub = (C*)c.d_ub;
     C* uz = (C*)c.d_uz;
-    const int kxn = c.g.kxn;
     k_yinv<T, N><<<dim3(c.nab_i, 3), K1Launch<T, N>::THREADS, sm1(), c.stream>>>(
         g, st, (const C*)(which == PSDNS_FIELD_U ? c.d_u : c.d_un), ub, tw);
-    k_zinv<T, N, 0, true><<<k2_grid(2), ZL::THREADS, sm2(),
-                           c.stream>>>(g, ub, uz, tw, st.b11, st.b33);
+    k_zinv<T, N, 0, true><<<k2_grid(2), ZL::THREADS, sm2(), c.stream>>>(g, ub, uz, tw, st.b11, st.b33);
     // the transposed copy in ub is consumed: its space holds the partial sums
     double* partial = (double*)c.d_ub;
     double* d_out = partial + (size_t)c.nzt * N * 16;
@@ -486,7 +482,8 @@ template <typename T, int N, int NC> struct Impl {
       double* d_tk = (double*)c.d_efkz;   // n/2 + 2 shells of 3 doubles: room for n/2
       if (cudaMemsetAsync(d_tk, 0, sizeof(double) * (N / 2), c.stream) != cudaSuccess) rc = set_error("memset");
       if (!rc) {
-        k_yfwd<T, N, 0, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), K5Launch<T, N, NC>::THREADS, sm5() + sizeof(double) * (N / 2), c.stream>>>(
+        k_yfwd<T, N, 0, NC><<<K5Launch<T, N, NC>::blocks(c.nab_f), K5Launch<T, N, NC>::THREADS,
+                              sm5() + sizeof(double) * (N / 2), c.stream>>>(
             g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, d_tk);
         if (cudaGetLastError() != cudaSuccess) rc = set_error("transfer launch failed");
       }
@@ -521,17 +518,18 @@ template <typename T, int N, int NC> struct Impl {
     C* u = (C*)c.d_u;
     C* ub = (C*)c.d_ub;
     C* uz = (C*)c.d_uz;
-    const int kxn = c.g.kxn;
     const int s = kstep - 1;
     {
       constexpr int TH = K1Launch<T, N>::THREADS;
       prof_mark(c, s, 0, 0);
-      launch_dep<DEP>(k_yinv<T, N, false, NC>, dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), TH, sm1(), c.stream, g, st, u, ub, tw, TcArgs());
+      launch_dep<DEP>(k_yinv<T, N, false, NC>, dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), TH, sm1(), c.stream, g, st, u,
+                      ub, tw, TcArgs());
       prof_mark(c, s, 0, 1);
     }
     {
       prof_mark(c, s, 1, 0);
-      launch_dep<DEP>(k_zinv<T, N, NC>, k2_grid(3 + 3 * NC), ZL::THREADS, sm2(), c.stream, g, ub, uz, tw, st.b11, st.b33, TcArgs());
+      launch_dep<DEP>(k_zinv<T, N, NC>, k2_grid(3 + 3 * NC), ZL::THREADS, sm2(), c.stream, g, ub, uz, tw, st.b11,
+                      st.b33, TcArgs());
       prof_mark(c, s, 1, 1);
     }
     {
@@ -540,21 +538,23 @@ template <typename T, int N, int NC> struct Impl {
       // mean-gradient coefficients cb = beta * grad (init.f:42-45)
       const T cb1 = (T)(c.p.beta1 * c.p.grad[0]), cb2 = (T)(c.p.beta2 * c.p.grad[1]),
               cb3 = (T)(c.p.beta3 * c.p.grad[2]);
-      launch_dep<DEP>(k_xchain<T, N, NC>, dim3(N / K3Launch<T, N, NC>::TZ, N), TH, sm3(), c.stream, g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1, cb2, cb3, TcArgs());
+      launch_dep<DEP>(k_xchain<T, N, NC>, dim3(N / K3Launch<T, N, NC>::TZ, N), TH, sm3(), c.stream, g, uz, tw, st.b11,
+                      st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1, cb2, cb3, TcArgs());
       prof_mark(c, s, 2, 1);
     }
     {
       prof_mark(c, s, 3, 0);
       const int tiles = k4_tiles(1);
-      launch_dep<DEP>(k_zfwd<T, N, NC>, k4_grid(tiles), ZL::THREADS, sm4(), c.stream, g, uz, ub, tw, tiles, st.b11, st.b33, TcArgs());
+      launch_dep<DEP>(k_zfwd<T, N, NC>, k4_grid(tiles), ZL::THREADS, sm4(), c.stream, g, uz, ub, tw, tiles, st.b11,
+                      st.b33, TcArgs());
       prof_mark(c, s, 3, 1);
     }
     CK(cudaGetLastError());
     return 0;
   }
 
-  // stage part A with the 1-D transforms on the tensor cores (same launch
-  // grids as stage_a)
+  // stage part A with the 1-D transforms on the tensor cores (K1 and K3 in the
+  // grids of stage_a, K2 a block per panel, K4 one per half a panel)
   static int stage_a_tc(Ctx& c, int kstep) {
     Geo g = make_geo(c);
     StageTables<T> st = make_tables<T>(c, (kstep - 1) & 1);
@@ -563,23 +563,21 @@ template <typename T, int N, int NC> struct Impl {
     C* u = (C*)c.d_u;
     C* ub = (C*)c.d_ub;
     C* uz = (C*)c.d_uz;
-    const int kxn = c.g.kxn;
     const int s = kstep - 1;
     prof_mark(c, s, 0, 0);
     k_yinv<T, N, false, NC, true><<<dim3(k1_blocks<T>(c.nab_i), 3 + 2 * NC), K1Launch<T, N>::THREADS,
                                     sm1tc(), c.stream>>>(g, st, u, ub, tw, ta);
     prof_mark(c, s, 0, 1);
     prof_mark(c, s, 1, 0);
-    k_zinv<T, N, NC, false, true><<<dim3(N, (kxn + kTcXT2 - 1) / kTcXT2, 3 + 3 * NC),
-                                            Launch<T, N, kTcXT2>::THREADS, sm2tc(), c.stream>>>(
+    k_zinv<T, N, NC, false, true><<<dim3(N, ZL::NPAN, 3 + 3 * NC), Launch<T, N, kTcXT2>::THREADS, sm2tc(), c.stream>>>(
         g, ub, uz, tw, st.b11, st.b33, ta);
     prof_mark(c, s, 1, 1);
     prof_mark(c, s, 2, 0);
     const T cb1 = (T)(c.p.beta1 * c.p.grad[0]), cb2 = (T)(c.p.beta2 * c.p.grad[1]),
             cb3 = (T)(c.p.beta3 * c.p.grad[2]);
-    k_xchain<T, N, NC, true><<<dim3(N / K3Launch<T, N, NC, true>::TZ, N), K3Launch<T, N, NC, true>::THREADS, K3Launch<T, N, NC, true>::SMEM_TC,
-                               c.stream>>>(g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1,
-                                           cb2, cb3, ta);
+    using K3 = K3Launch<T, N, NC, true>;
+    k_xchain<T, N, NC, true><<<dim3(N / K3::TZ, N), K3::THREADS, K3::SMEM_TC, c.stream>>>(
+        g, uz, tw, st.b11, st.b22, st.b33, c.d_velmax, kstep == 1 ? 1 : 0, cb1, cb2, cb3, ta);
     prof_mark(c, s, 2, 1);
     prof_mark(c, s, 3, 0);
     k_zfwd<T, N, NC, true><<<dim3(N * (Panel<T, N>::PW / kTcXT4), ZL::NPAN),
@@ -607,22 +605,25 @@ template <typename T, int N, int NC> struct Impl {
     return 0;
   }
 
-  // stage part B: K5
+  // stage part B: K5 (one slot of columns a block or two, K5Launch)
+  template <typename K>
+  static void launch_k5(Ctx& c, int kstep, K kernel, C* racc) {
+    using K5 = K5Launch<T, N, NC>;
+    launch_dep<DEP>(kernel, K5::blocks(c.nab_f), K5::THREADS, sm5(), c.stream, make_geo(c),
+                    make_tables<T>(c, (kstep - 1) & 1), (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw,
+                    c.d_efkz, TcArgs(), racc);
+  }
+
   // K5 of the RK4 sub-stages (velocity only)
   static int stage_b_rk4(Ctx& c, int kstep) {
     if constexpr (NC == 0) {
-      Geo g = make_geo(c);
-      StageTables<T> st = make_tables<T>(c, (kstep - 1) & 1);
-      constexpr int TH = K5Launch<T, N, NC>::THREADS;
-      const C* ub = (const C*)c.d_ub;
-      C *u = (C*)c.d_u, *un = (C*)c.d_un, *r = (C*)c.d_u1;
-      const C* tw = (const C*)c.d_tw;
+      C* r = (C*)c.d_u1;
       prof_mark(c, kstep - 1, 4, 0);
       switch (kstep) {
-        case 1: launch_dep<DEP>(k_yfwd<T, N, 11>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 2: launch_dep<DEP>(k_yfwd<T, N, 12>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        case 3: launch_dep<DEP>(k_yfwd<T, N, 13>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r); break;
-        default: launch_dep<DEP>(k_yfwd<T, N, 14>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, ub, u, un, tw, c.d_efkz, TcArgs(), r);
+        case 1: launch_k5(c, kstep, k_yfwd<T, N, 11>, r); break;
+        case 2: launch_k5(c, kstep, k_yfwd<T, N, 12>, r); break;
+        case 3: launch_k5(c, kstep, k_yfwd<T, N, 13>, r); break;
+        default: launch_k5(c, kstep, k_yfwd<T, N, 14>, r);
       }
       prof_mark(c, kstep - 1, 4, 1);
       CK(cudaGetLastError());
@@ -636,14 +637,11 @@ template <typename T, int N, int NC> struct Impl {
     if (c.rk == 4) return stage_b_rk4(c, kstep);
     if constexpr (kTc)
       if (c.dft == PSDNS_DFT_TC_BF16X3) return stage_b_tc(c, kstep);
-    Geo g = make_geo(c);
-    StageTables<T> st = make_tables<T>(c, (kstep - 1) & 1);
-    constexpr int TH = K5Launch<T, N, NC>::THREADS;
     prof_mark(c, kstep - 1, 4, 0);
     if (kstep == 1)
-      launch_dep<DEP>(k_yfwd<T, N, 1, NC>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, TcArgs(), (C*)nullptr);
+      launch_k5(c, kstep, k_yfwd<T, N, 1, NC>, (C*)nullptr);
     else
-      launch_dep<DEP>(k_yfwd<T, N, 2, NC>, K5Launch<T, N, NC>::blocks(c.nab_f), TH, sm5(), c.stream, g, st, (const C*)c.d_ub, (C*)c.d_u, (C*)c.d_un, (const C*)c.d_tw, c.d_efkz, TcArgs(), (C*)nullptr);
+      launch_k5(c, kstep, k_yfwd<T, N, 2, NC>, (C*)nullptr);
     prof_mark(c, kstep - 1, 4, 1);
     CK(cudaGetLastError());
     return 0;
@@ -1283,7 +1281,8 @@ int psdns_gpu_init(const psdns_params* p, void** out) {
   // ub: 3 + 2 nc backward variables (TB_I blocks) or 4 + nc forward terms
   // (TB_F blocks); uz: 5 + nc slots (3 + 3 nc inputs, 5 + nc outputs)
   const size_t ubi = dbl ? ubi_var_elems<double>(c->nab_i, n) : ubi_var_elems<float>(c->nab_i, n);
-  c->ub_elems = std::max((size_t)(3 + 2 * c->nc) * ubi, (size_t)(4 + c->nc) * (dbl ? ubf_var_elems<double>(c->nab_f, n) : ubf_var_elems<float>(c->nab_f, n)));
+  const size_t ubf = dbl ? ubf_var_elems<double>(c->nab_f, n) : ubf_var_elems<float>(c->nab_f, n);
+  c->ub_elems = std::max((size_t)(3 + 2 * c->nc) * ubi, (size_t)(4 + c->nc) * ubf);
   c->uz_elems = (size_t)(5 + c->nc) * n * (dbl ? uz_slab<double>(n) : uz_slab<float>(n));
   c->st_elems = (size_t)c->nv * c->g.xz_tot * n;
   c->rng.init(p->seed_input);

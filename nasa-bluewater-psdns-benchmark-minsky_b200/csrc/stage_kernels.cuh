@@ -176,10 +176,15 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // (__ldg, or a const __restrict__ kernel parameter), which is for the geometry and
 // the tables.
 // dep_launch: boxes of n <= 128 without a scalar, whose kernels are about as
-// short as the gaps between them (step of 64^3 FP32 118 -> 107 us, 128^3 235 ->
-// 221).  Where a kernel fills the GPU many times over, the blocks that wait
-// disturb it: 1024^3 64.0 -> 70.2 ms, 512^3 7.9 -> 8.5, 256^3 with a scalar and
-// particles 1.66 -> 1.71.
+// short as the gaps between them.  Steps without -> with it: FP32 16^3 85 -> 81 us,
+// 32^3 97 -> 89, 48^3 96 -> 90, 64^3 108 -> 97, 128^3 218 -> 205, but 96^3 160 ->
+// 165; FP64 16^3 89 -> 80, 32^3 102 -> 96, 128^3 338 -> 322, 64^3 and 96^3 the
+// same, 48^3 111 -> 115.  With a scalar: FP32 64^3 113 -> 105 and 128^3 277 -> 266,
+// but 48^3 117 -> 122, 96^3 206 -> 211 and FP64 64^3 138 -> 141, 96^3 309 -> 311.
+// Where a kernel fills the GPU many times over, the blocks that wait disturb it:
+// 1024^3 64.0 -> 70.2 ms, 512^3 7.9 -> 8.5, 256^3 with a scalar and particles
+// 1.66 -> 1.71.  The particle chain, whose spline and gather kernels have no
+// dep_wait, is launched plainly at every n; it was not measured the other way.
 __host__ __device__ constexpr bool dep_launch(int n, int nc) { return n <= 128 && nc == 0; }
 __device__ __forceinline__ void dep_wait() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -226,7 +231,7 @@ __device__ __forceinline__ void load_twiddles(C2<T>* tw_s, const C2<T>* __restri
 }
 
 // threads of a block that transforms LINES lines at once (capped at CAP, at
-// least one warp, and a multiple of the P threads of a line: P = 6 at
+// least one warp, and a multiple of the P threads of a line: P = 4 at
 // n = 48)
 __host__ __device__ constexpr int round_up(int a, int m) { return (a + m - 1) / m * m; }
 __host__ __device__ constexpr int gcd_c(int a, int b) { return b == 0 ? a : gcd_c(b, a % b); }
@@ -545,7 +550,9 @@ k_zinv(Geo g, const C2<T>* ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__
     tc::fft1024<THREADS>(
         XT, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * L * sizeof(C)), begin,
         [&](const Line& s, int z) { return fix(s, z, fetch(s, z)); }, [&](int l) { return (unsigned)l * 16; },
-        [&](unsigned o, int z, C val) { *reinterpret_cast<C*>(panel + (PA::template off<false>(z) ^ o)) = cconj(val); });
+        [&](unsigned o, int z, C val) {
+          *reinterpret_cast<C*>(panel + (PA::template off<false>(z) ^ o)) = cconj(val);
+        });
     tc::teardown<NCOL>(w);
     panel_to_global(plane + (size_t)blockIdx.y * PA::ELEMS, panel, PA::BYTES);
   } else {
@@ -567,7 +574,8 @@ k_zinv(Geo g, const C2<T>* ub, C2<T>* __restrict__ uz, const C2<T>* __restrict__
 #pragma unroll
           for (int r = 0; r < H; r++) {
             const bool in = h == 0 ? z0 + r * S0 <= s.kc : z0 + r * S0 >= -s.kc;
-            val[q * R0 + h * H + r] = in ? ld_step<dep_launch(N, NC)>(p0 + (long)r * ((long)(S0 / TBL) * N * TBL)) : cmk<C>(0, 0);
+            val[q * R0 + h * H + r] =
+                in ? ld_step<dep_launch(N, NC)>(p0 + (long)r * ((long)(S0 / TBL) * N * TBL)) : cmk<C>(0, 0);
           }
         }
     } else {
@@ -1055,11 +1063,9 @@ __device__ __forceinline__ void zfwd_store(const Geo& g, const C2<T>* s0, const 
       const T bk1 = b11 * T(x), kz = T(kwave<N>(z));
       const C p3 = s1[i], p5 = s0[i];
       out = cmk<C>(-bk1 * p5.y - kz * p3.y, bk1 * p5.x + kz * p3.x);
-    } else if constexpr (MODE == 2) {
-      out = s0[i];
-    } else if constexpr (MODE == 3) {
+    } else if constexpr (MODE == 2) {   // the scalar's term
       out = s1[i];
-    } else {                            // MODE 4: s0 to this slot and s1 to slot + 2
+    } else {                            // MODE 3: s0 to this slot and s1 to slot + 2
       out = s0[i];
       dst[2 * ubf_var_elems<T>(g.nab_f, N) + ((size_t)((unsigned)a / TB) * N + y0) * TB + (((unsigned)a % TB) ^ swap)] =
           s1[i];
@@ -1273,14 +1279,14 @@ k_zfwd(Geo g, const C2<T>* uz, C2<T>* __restrict__ ub, const C2<T>* __restrict__
     __syncthreads();
     both();
     // P2 -> ub slot 1 and P4 -> ub slot 3 in one pass over the cylinder indices
-    zfwd_store<T, N, 4, XT>(g, s0, s1, L, ub, 1, y, x0, x1, b11, b33);
+    zfwd_store<T, N, 3, XT>(g, s0, s1, L, ub, 1, y, x0, x1, b11, b33);
     if constexpr (NC > 0) {
       __syncthreads();
       zfwd_load<T, N, THREADS>(uz, 5, y, x0, nl, s1, L);
       cp_async_wait_all();
       __syncthreads();
       lines_fft<T, N, THREADS, TCM>(s1, nl, L, tw, w);
-      zfwd_store<T, N, 3, XT>(g, s0, s1, L, ub, 4, y, x0, x1, b11, b33);
+      zfwd_store<T, N, 2, XT>(g, s0, s1, L, ub, 4, y, x0, x1, b11, b33);
     }
     tc::teardown<NCOL>(w);
   }
@@ -1337,7 +1343,8 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* ub, C2<T>* __restrict__ u,
   using KL = K5Launch<T, N, NC>;
   using PA = typename KL::PA;
   constexpr bool PAD = TCM || !KL::SLOT;   // padded lines, else one-slot panels
-  constexpr int SC = Tiles<T>::TB_F, SPB = TCM ? KL::SPB_TC : KL::SPB, TB = SPB * SC, TBL = Tiles<T>::TBL_F, R = TBL / SC;
+  constexpr int SC = Tiles<T>::TB_F, SPB = TCM ? KL::SPB_TC : KL::SPB, TB = SPB * SC;
+  constexpr int TBL = Tiles<T>::TBL_F, R = TBL / SC;
   static_assert(R % SPB == 0, "a block's slots lie in one run");
   constexpr int NVF = 4 + NC;
   constexpr int THREADS = TCM ? KL::THREADS_TC : KL::THREADS;
@@ -1371,10 +1378,9 @@ k_yfwd(Geo g, StageTables<T> st_all, const C2<T>* ub, C2<T>* __restrict__ u,
   // threads divide a column, a step stays inside it
   constexpr int PER = (TB * N + THREADS - 1) / THREADS;
   constexpr bool DIV = N % THREADS == 0;
-  auto col_of = [&](int q) { return DIV ? q / (N / THREADS > 0 ? N / THREADS : 1) : ((int)threadIdx.x + q * THREADS) / N; };
-  auto row_of = [&](int q) {
-    return DIV ? (int)threadIdx.x + q % (N / THREADS > 0 ? N / THREADS : 1) * THREADS : ((int)threadIdx.x + q * THREADS) % N;
-  };
+  constexpr int QC = N / THREADS > 0 ? N / THREADS : 1;   // steps of a column, where DIV
+  auto col_of = [&](int q) { return DIV ? q / QC : ((int)threadIdx.x + q * THREADS) / N; };
+  auto row_of = [&](int q) { return DIV ? (int)threadIdx.x + q % QC * THREADS : ((int)threadIdx.x + q * THREADS) % N; };
   // un is read after the transform (its registers are free then): bring the
   // sphere's part of it into L2 meanwhile
   if constexpr (!TCM) {

@@ -185,25 +185,22 @@ static int run(const psdns_params* prm, int kstep, const double* gsh, double dt,
   C* uz = (C*)(base + pl.uz);
   const C* twd = (const C*)(base + pl.tw);
   unsigned long long* vmx = (unsigned long long*)(base + pl.velmax);
-  {
-    constexpr int TH = K1Launch<T, N>::THREADS;
-    launch_dep<dep_launch(N, 0)>(k_yinv<T, N>, dim3(k1_blocks<T>(geo.nab_i), 3), TH, K1Launch<T, N>::SMEM, st, geo, stb, u, ub, twd, TcArgs());
-  }
+  constexpr bool DEP = dep_launch(N, 0);
+  using K1 = K1Launch<T, N>;
   using ZL = ZLaunch<T, N, 0>;
-  launch_dep<dep_launch(N, 0)>(k_zinv<T, N>, dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st, geo, ub, uz, twd, T(1), T(1), TcArgs());
-  {
-    constexpr int TH = K3Launch<T, N, 0>::THREADS;
-    launch_dep<dep_launch(N, 0)>(k_xchain<T, N>, dim3(N / K3Launch<T, N, 0>::TZ, N), TH, K3Launch<T, N, 0>::SMEM, st, geo, uz, twd, stb.b11, stb.b22, stb.b33, vmx, kstep == 1 ? 1 : 0, T(0), T(0), T(0), TcArgs());
-  }
+  using K3 = K3Launch<T, N, 0>;
+  using K5 = K5Launch<T, N, 0>;
   const int tiles = N * ZL::TILES;
-  launch_dep<dep_launch(N, 0)>(k_zfwd<T, N>, std::min(tiles, 148 * ZL::MINB4), ZL::THREADS, ZL::SMEM4, st, geo, uz, ub, twd, tiles, stb.b11, stb.b33, TcArgs());
-  {
-    constexpr int TH = K5Launch<T, N, 0>::THREADS;
-    if (kstep == 1)
-      launch_dep<dep_launch(N, 0)>(k_yfwd<T, N, 1>, K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st, geo, stb, ub, u, un, twd, (double*)nullptr, TcArgs(), (C*)nullptr);
-    else
-      launch_dep<dep_launch(N, 0)>(k_yfwd<T, N, 2>, K5Launch<T, N, 0>::blocks(geo.nab_f), TH, K5Launch<T, N, 0>::SMEM, st, geo, stb, ub, u, un, twd, (double*)nullptr, TcArgs(), (C*)nullptr);
-  }
+  launch_dep<DEP>(k_yinv<T, N>, dim3(k1_blocks<T>(geo.nab_i), 3), K1::THREADS, K1::SMEM, st, geo, stb, u, ub, twd,
+                  TcArgs());
+  launch_dep<DEP>(k_zinv<T, N>, dim3(N, ZL::TILES, 3), ZL::THREADS, ZL::SMEM2, st, geo, ub, uz, twd, T(1), T(1),
+                  TcArgs());
+  launch_dep<DEP>(k_xchain<T, N>, dim3(N / K3::TZ, N), K3::THREADS, K3::SMEM, st, geo, uz, twd, stb.b11, stb.b22,
+                  stb.b33, vmx, kstep == 1 ? 1 : 0, T(0), T(0), T(0), TcArgs());
+  launch_dep<DEP>(k_zfwd<T, N>, std::min(tiles, 148 * ZL::MINB4), ZL::THREADS, ZL::SMEM4, st, geo, uz, ub, twd, tiles,
+                  stb.b11, stb.b33, TcArgs());
+  launch_dep<DEP>(kstep == 1 ? k_yfwd<T, N, 1> : k_yfwd<T, N, 2>, K5::blocks(geo.nab_f), K5::THREADS, K5::SMEM, st, geo,
+                  stb, ub, u, un, twd, (double*)nullptr, TcArgs(), (C*)nullptr);
   NA_CK(cudaGetLastError());
   unsigned long long vm_bits = 0;
   if (kstep == 1) NA_CK(cudaMemcpyAsync(&vm_bits, vmx, sizeof vm_bits, cudaMemcpyDeviceToHost, st));

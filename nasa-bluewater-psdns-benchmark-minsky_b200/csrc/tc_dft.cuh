@@ -365,7 +365,8 @@ __device__ __forceinline__ void fft1024_lines(float2* buf, int nlines, int ls, W
   auto line = [&](int l) { return buf + (size_t)l * ls; };
   fft1024<THREADS>(
       nlines, w, reinterpret_cast<unsigned char*>(buf), (uint32_t)(4 * ls * sizeof(float2)), line,
-      [](const float2* p, int i) { return p[padl<float2, 1024>(i)]; }, line, [](float2* p, int k, float2 v) { p[padl<float2, 1024>(k)] = v; });
+      [](const float2* p, int i) { return p[padl<float2, 1024>(i)]; }, line,
+      [](float2* p, int k, float2 v) { p[padl<float2, 1024>(k)] = v; });
   __syncthreads();
 }
 
