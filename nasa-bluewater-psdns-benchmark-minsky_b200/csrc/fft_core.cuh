@@ -19,7 +19,7 @@
 // What bounds the transforms inside the kernels is the number of instructions
 // issued, not the FMA pipe (with scalar arithmetic and the twiddles multiplied
 // onto the operands the x chain issued 0.59 per cycle and scheduler at 40% of that
-// pipe; in this form 0.60, in a quarter fewer instructions: 914 -> 672 million a
+// pipe; in this form 0.61, in a quarter fewer instructions: 914 -> 690 million a
 // launch at 512^3 FP32), so the arithmetic is arranged for few instructions:
 //  * Complex sums, and the sums of a twiddled butterfly, are packed FP32 pair
 //    instructions (add, subtract, fma of (re, im)): one issue slot instead of
